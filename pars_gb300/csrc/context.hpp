@@ -444,6 +444,7 @@ struct batch_job_device
   int                 ux, uy, uz;     // lattice seeds: output voxel shape (0 = output per seed)
   float4*             end_positions;  // may be nullptr
   int*                end_steps;      // may be nullptr
+  int                 pool;           // seeds per pool (batch_pool_for)
   long long           first_pool;     // pools of all earlier jobs
   unsigned long long* steps;          // per-job step counter
 };
@@ -453,7 +454,8 @@ int  batch_variant_count();
 // Resident warps per SM of a job class's launch shape.
 int  batch_resident_warps(pars_gpu_context& ctx, int job_class, int variant);
 int  batch_variant_threads(int variant);
-int  batch_pool_seeds();
+// Seeds per pool for a launch (or a job) of `seeds` seeds.
+int  batch_pool_for(pars_gpu_context& ctx, int job_class, int variant, long long seeds);
 // job_class: batch_steady, batch_unsteady or batch_frozen.
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int variant, const batch_job_device* jobs, int njobs,
                          long long total_chunks, unsigned long long* counter);
