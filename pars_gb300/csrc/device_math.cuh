@@ -30,8 +30,25 @@ struct field_view
   float         ox, oy, oz;        // offset
   float         hx, hy, hz;        // spacing
   float         maxx, maxy, maxz;  // offset + size (block-exit face tests)
-  float         inv_hx, inv_hy, inv_hz;  // 1 / spacing (re-sampled path)
+  float         inv_hx, inv_hy, inv_hz;  // RN(1 / spacing)
+  int           fast_division;           // 1: quotient_rn holds for this spacing (divides_fast)
 };
+
+// Whether x / h may be formed with quotient_rn for this spacing: with h in
+// [2^-20, 2^20] and |x| >= 2^-63 (or x = +0) no step of it leaves the normal
+// range but the remainder, which stays exact.
+inline bool divides_fast(float hx, float hy, float hz)
+{
+  auto in = [](float h) { return h >= 0x1p-20f && h <= 0x1p20f; };
+  return in(hx) && in(hy) && in(hz);
+}
+
+// Reciprocals and the division flag of a view whose spacing is set.
+inline void set_reciprocals(field_view& f)
+{
+  f.inv_hx = 1.0f / f.hx; f.inv_hy = 1.0f / f.hy; f.inv_hz = 1.0f / f.hz;
+  f.fast_division = divides_fast(f.hx, f.hy, f.hz) ? 1 : 0;
+}
 
 // The termination and invalid vertices (integral_curves.hpp:18-19).
 __device__ __forceinline__ float4 termination_vertex() { return make_float4(-2.0f, -2.0f, -2.0f, 0.0f); }
@@ -67,6 +84,52 @@ __device__ __forceinline__ axis_cell cell_of(float p, float o, float h)
   if (d >= 0.0f) { if (r < 0.0f) r = __fmaf_rn(-(s - 1.0f), h, d); }
   else           { if (r > 0.0f) r = __fmaf_rn(-(s + 1.0f), h, d); }
   return axis_cell{s, __fdiv_rn(r, h)};
+}
+
+// RN(x / h) from y = RN(1 / h): the product x y, corrected by its exact FMA
+// remainder (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990).  q = RN(x y) is within 1.5
+// ulp of x / h, so q + r y misses x / h by at most 1.5 2^-25 h ulps (h scaled to
+// [1, 2)), and rounds wrongly only where x / h lies that close to the midpoint
+// of two floats.  Those pairs are few -- a quotient of 24-bit significands X / H
+// near an odd multiple of half an ulp solves M H = X 2^c + e with |e| <= 2 -- and
+// all 23 M of them (|e| <= 4, every H) give RN(x / h).  Three instructions and no
+// special cases; the hardware-assisted division sequence costs about ten.
+__device__ __forceinline__ float quotient_rn(float x, float h, float y)
+{
+  const float q = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-q, h, x), y, q);
+}
+
+// cell_of for a spacing with fast_division and |d| >= 2^-40 (so that the
+// remainder is 0 or at least 2^-63) or d = +0: the same values.
+__device__ __forceinline__ axis_cell cell_of_fast(float d, float h, float y)
+{
+  const float s = floorf(quotient_rn(d, h, y));
+  float r = __fmaf_rn(-s, h, d);
+  if (d >= 0.0f) { if (r < 0.0f) r = __fmaf_rn(-(s - 1.0f), h, d); }
+  else           { if (r > 0.0f) r = __fmaf_rn(-(s + 1.0f), h, d); }
+  return axis_cell{s, quotient_rn(r, h, y)};
+}
+
+// cell_of on the three axes.
+__device__ __forceinline__ void cells_of(const field_view& f, const float4& p, axis_cell& cx, axis_cell& cy, axis_cell& cz)
+{
+  const float dx = __fsub_rn(p.x, f.ox), dy = __fsub_rn(p.y, f.oy), dz = __fsub_rn(p.z, f.oz);
+  // bits of |d|, +0 (the grid's first planes) apart
+  auto fits = [](float d) { return fabsf(d) >= 0x1p-40f || __float_as_uint(d) == 0u; };
+  if (f.fast_division && fits(dx) && fits(dy) && fits(dz))
+  {
+    cx = cell_of_fast(dx, f.hx, f.inv_hx);
+    cy = cell_of_fast(dy, f.hy, f.inv_hy);
+    cz = cell_of_fast(dz, f.hz, f.inv_hz);
+  }
+  else
+  {
+    cx = cell_of(p.x, f.ox, f.hx);
+    cy = cell_of(p.y, f.oy, f.hy);
+    cz = cell_of(p.z, f.oz, f.hz);
+  }
 }
 
 __device__ __forceinline__ bool cell_inside(float s, int n) { return s >= 0.0f && s <= float(n - 2); }
@@ -120,9 +183,8 @@ __device__ __forceinline__ float3 gather_blend(const field_view& f, int ix, int 
 // contains() followed by interpolate() at p: returns false when p is outside.
 __device__ __forceinline__ bool sample_inside(const field_view& f, const float4& p, float3& v)
 {
-  const axis_cell cx = cell_of(p.x, f.ox, f.hx);
-  const axis_cell cy = cell_of(p.y, f.oy, f.hy);
-  const axis_cell cz = cell_of(p.z, f.oz, f.hz);
+  axis_cell cx, cy, cz;
+  cells_of(f, p, cx, cy, cz);
   if (!(cell_inside(cx.s, f.nx) && cell_inside(cy.s, f.ny) && cell_inside(cz.s, f.nz))) return false;
   v = gather_blend(f, int(cx.s), int(cy.s), int(cz.s), cx.w, cy.w, cz.w);
   return true;
@@ -205,9 +267,8 @@ __device__ __forceinline__ float3 blend8_cached(const corner_cache& k, float wx,
 // blend), the cell's corners kept in the lane's cache between steps.
 __device__ __forceinline__ bool sample_inside_cached(const field_view& f, corner_cache& k, const float4& p, float3& v)
 {
-  const axis_cell cx = cell_of(p.x, f.ox, f.hx);
-  const axis_cell cy = cell_of(p.y, f.oy, f.hy);
-  const axis_cell cz = cell_of(p.z, f.oz, f.hz);
+  axis_cell cx, cy, cz;
+  cells_of(f, p, cx, cy, cz);
   if (!(cell_inside(cx.s, f.nx) && cell_inside(cy.s, f.ny) && cell_inside(cz.s, f.nz))) return false;
   const int ix = int(cx.s), iy = int(cy.s), iz = int(cz.s);
   if (ix != k.ix || iy != k.iy || iz != k.iz) corner_load(f, k, ix, iy, iz);
@@ -259,7 +320,11 @@ __device__ __forceinline__ bool is_zero(const float3& v)
 //  * Adams-Bashforth 2: the particle's first step is the weighted sum (RK4
 //    weights), later ones out = x + c_4 v_n + c_5 v_{n-1} (c_4 = 1.5 h,
 //    c_5 = -0.5 h), with the previous step's velocity kept per particle.
-enum frozen_method { frozen_weighted_sum = 0, frozen_midpoint = 1, frozen_multistep = 2 };
+//  * RK4, the weighted sum with c_0 = c_3 and c_1 = c_2, is its own method: two
+//    products per component instead of four, no loop.
+enum frozen_method { frozen_weighted_sum = 0, frozen_midpoint = 1, frozen_multistep = 2, frozen_rk4 = 3 };
+
+
 
 // Re-sampled stages of the other integrators ("true form"): explicit RK
 // tableaux (modified midpoint as a 3-stage scheme, Cash-Karp 5(4) and
@@ -300,10 +365,20 @@ __device__ __forceinline__ float multistep_component(const step_rule& r, float x
   return __fadd_rn(__fadd_rn(x, __fmul_rn(r.c[4], v)), __fmul_rn(r.c[5], previous));
 }
 
+__device__ __forceinline__ float rk4_component(const step_rule& r, float x, float v)
+{
+  const float a = __fmul_rn(r.c[0], v), b = __fmul_rn(r.c[1], v);
+  return __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(x, a), b), b), a);
+}
+
 // FROZEN step from x with the velocity v = v(x): the reference's operation order.
 __device__ __forceinline__ float4 frozen_step(const step_rule& r, const float4& x, const float3& v, frozen_history& hist)
 {
   float4 out;
+  if (r.method == frozen_rk4)
+    // w: adding c 0 = +-0 four times is adding it once
+    return make_float4(rk4_component(r, x.x, v.x), rk4_component(r, x.y, v.y), rk4_component(r, x.z, v.z),
+                       __fadd_rn(x.w, __fmul_rn(r.c[0], 0.0f)));
   if (r.method == frozen_midpoint)
     out = make_float4(midpoint_component(r, x.x, v.x), midpoint_component(r, x.y, v.y), midpoint_component(r, x.z, v.z),
                       midpoint_component(r, x.w, 0.0f));

@@ -359,7 +359,7 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   f.ox = offset[0]; f.oy = offset[1]; f.oz = offset[2];
   f.hx = spacing[0]; f.hy = spacing[1]; f.hz = spacing[2];
   f.maxx = offset[0] + size[0]; f.maxy = offset[1] + size[1]; f.maxz = offset[2] + size[2];
-  f.inv_hx = 1.0f / spacing[0]; f.inv_hy = 1.0f / spacing[1]; f.inv_hz = 1.0f / spacing[2];
+  set_reciprocals(f);
 
   // The counter keeps the previous call's value: clear it first.
   if (cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }

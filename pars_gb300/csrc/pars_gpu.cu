@@ -296,7 +296,10 @@ step_rule make_rule(int integrator, int stage_mode, float h)
     r.c[5] = weight_times(-1, 2, h);
     break;
   case PARS_ADAMS_BASHFORTH_MOULTON_2: weights({{1, 2}, {1, 2}}); break;
-  default: weights({{1, 6}, {1, 3}, {1, 3}, {1, 6}}); break;    // RK4
+  default:
+    weights({{1, 6}, {1, 3}, {1, 3}, {1, 6}});           // RK4
+    r.method = frozen_rk4;
+    break;
   }
   return r;
 }
