@@ -246,6 +246,7 @@ struct pars_gpu_context
   // and the device's SM count, queried once
   int                                     trace_ctas_per_sm[3] = {-1, -1, -1};
   int                                     async_ctas_per_sm[3] = {-1, -1, -1};
+  int                                     flow_map_ctas[8] = {-1, -1, -1, -1, -1, -1, -1, -1};   // per-seed flow maps: resident CTAs by scheme
   int                                     sm_count = 0;
   // batched engine: resident CTAs per SM per job class and launch shape
   int                                     batch_ctas_per_sm[3][4] = {{-1, -1, -1, -1}, {-1, -1, -1, -1}, {-1, -1, -1, -1}};
@@ -524,9 +525,10 @@ void trace_rounds(pars_gpu_context& ctx, const std::vector<trace_block>& blocks,
 std::vector<unsigned long long> run_batch(pars_gpu_context& ctx, std::vector<batch_job_device>& jobs, int variant);
 pars_partition_info partition(int ranks, int rank, const int32_t domain[3]);
 
-void launch_flow_map(pars_gpu_context& ctx, const field_view& f, const step_rule& rule, int iterations,
-                     const float offset[3], const float fm_spacing[3], const int seeds_per_dimension[3],
-                     const int fm_shape[3], float4* flow, unsigned long long* steps);
+// Returns the device counter of the steps taken (in ctx.counters).
+const unsigned long long* launch_flow_map(pars_gpu_context& ctx, const field_view& f, const step_rule& rule, int iterations,
+                                          const float offset[3], const float fm_spacing[3], const int seeds_per_dimension[3],
+                                          const int fm_shape[3], float4* flow);
 void launch_ftle(pars_gpu_context& ctx, const field_view& flow, double time, int mode, float* out);
 
 // Ray tracer (render_kernels.cu).

@@ -1,6 +1,6 @@
 // Flow-map advection and the fused FTLE kernel.
 //
-// flow map: one thread per seed of flow_map_generator's lattice
+// flow map: one particle per seed of flow_map_generator's lattice
 //   (flow_map_generator.cpp:23-43 + seed_generator.cpp:9-21, seeds generated in
 //   the kernel from the voxel index), advected with particle_advector's rules
 //   (particle_advector.cpp:74-139, one block: a particle stops with its current
@@ -21,6 +21,8 @@
 //   of its FP32 rate, and FP64 evaluation made this kernel FP64-pipe bound.
 //   The fractional-anisotropy mode (ftle_map_generator.cpp:51-54) needs no
 //   eigen-solve: it is evaluated from the invariants of C.
+#include <algorithm>
+
 #include "context.hpp"
 
 namespace pars
@@ -38,55 +40,168 @@ struct flow_map_args
   int        fx, fy, fz;          // flow-map shape
   float4*    flow;
   unsigned long long* steps;
+  unsigned long long* next;       // pool counter (zero before the launch)
 };
 
-template <bool FROZEN>
-__global__ void __launch_bounds__(256) flow_map_kernel(const __grid_constant__ flow_map_args a)
+// The stepping scheme a flow-map kernel is compiled for.
+enum flow_scheme { flow_frozen = 0, flow_classic, flow_midpoint, flow_cash_karp, flow_dormand_prince, flow_fehlberg,
+                   flow_adams_bashforth, flow_adams_moulton, flow_schemes };
+
+flow_scheme flow_scheme_of(const step_rule& r)
+{
+  if (r.frozen) return flow_frozen;
+  switch (r.scheme)
+  {
+  case scheme_tableau:         return flow_scheme(flow_midpoint + r.tableau);
+  case scheme_adams_bashforth: return flow_adams_bashforth;
+  case scheme_adams_moulton:   return flow_adams_moulton;
+  default:                     return flow_classic;
+  }
+}
+
+template <int SCHEME>
+__device__ __forceinline__ void flow_step(const flow_map_args& a, corner_cache& cache, local_position& q, const float3& v, frozen_history& hist)
+{
+  if constexpr (SCHEME == flow_classic)              local_step(a.f, cache, a.rule.rk4, a.rule.h, q, v);
+  else if constexpr (SCHEME == flow_adams_bashforth) adams_step_local<false>(a.f, cache, a.rule.h, q, v, hist);
+  else if constexpr (SCHEME == flow_adams_moulton)   adams_step_local<true>(a.f, cache, a.rule.h, q, v, hist);
+  else                                               tableau_step_local<SCHEME - flow_midpoint>(a.f, cache, a.rule.h, q, v);
+}
+
+// One particle per lane, and lanes whose particles have ended take the next
+// seeds of their warp's pool (refill_rule): particles leave the grid
+// after very different step counts, and with one seed per thread a warp's lanes
+// idled until its longest particle ended.  Warps take pools of `pool`
+// consecutive seeds from a device counter.  Bound by instruction issue and the
+// corner loads' L1 wavefronts, as the batched engine.  One seed per thread
+// against this: 5.51 -> 4.99 ms (frozen RK4, 150 x 128 x 141, 300 steps),
+// 657 -> 619 us (re-sampled RK4, 61 x 64 x 67, 120 steps, whole call).
+// Frozen steps need few registers once the corners are cached: seven CTAs of 128
+// per SM (72 registers) took 4.0 ms where 80 registers took 4.3 and 94 took 4.4
+// (150 x 128 x 141 vertices, 300 steps).  RK4 / Euler and Adams: five (96
+// registers); the tableaux keep what the compiler chooses (95 to 112).
+constexpr int flow_min_ctas(int scheme)
+{
+  return scheme == flow_frozen ? 7 : scheme == flow_classic || scheme >= flow_adams_bashforth ? 5 : 1;
+}
+
+template <int SCHEME>
+__global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(const __grid_constant__ flow_map_args a, int pool, refill_rule refill)
+{
+  constexpr unsigned full = 0xffffffffu;
+  const long long total = (long long)a.px * a.py * a.pz;
+  const int lane = threadIdx.x & 31;
+  const unsigned lanes_below = (1u << lane) - 1u;
+  long long pool_next = 0, pool_end = 0;   // warp-uniform
+  bool exhausted = false, alive = false, ended = false;   // ended: holds a particle not yet written
+  unsigned int steps = 0;                  // this lane's steps, all its particles
+  long long out = 0;                       // the particle's voxel, -1: none
+  int it = 1;
+  float4 pos = make_float4(0.f, 0.f, 0.f, 0.f);
+  local_position q {0, 0, 0, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  corner_cache cache;
+  frozen_history hist;
+  for (;;)
+  {
+    unsigned need = __ballot_sync(full, !alive);
+    if (__popc(need) >= (exhausted ? 32 : refill.lanes))
+    {
+      // write the ended particles, then give every idle lane a seed
+      if (ended)
+      {
+        // With iterations <= 1 the reference never assigns the voxel; it keeps the
+        // seed position here.
+        if constexpr (SCHEME != flow_frozen) { if (it > 1) pos = flow_position(a.f, q); }
+        if (out >= 0) a.flow[out] = pos;
+        ended = false;
+      }
+      while (need && !exhausted)
+      {
+        if (pool_next < pool_end)
+        {
+          const long long s = pool_next + __popc(need & lanes_below);
+          if (!alive && s < pool_end)
+          {
+            int ix, iy, iz;
+            lattice_index(s, a.py, a.pz, ix, iy, iz);
+            out = ix < a.fx && iy < a.fy && iz < a.fz ? ((long long)ix * a.fy + iy) * a.fz + iz : -1;
+            pos = make_float4(__fadd_rn(a.ox, __fmul_rn(a.sx, float(ix))), __fadd_rn(a.oy, __fmul_rn(a.sy, float(iy))),
+                              __fadd_rn(a.oz, __fmul_rn(a.sz, float(iz))), 0.0f);
+            hist = frozen_history();
+            // Re-sampled schemes in local cell coordinates (cell + offset +
+            // compensation); the position leaves them once, at the end.
+            if constexpr (SCHEME != flow_frozen) q = to_local(a.f, pos);
+            it = 1;
+            alive = true;
+          }
+          pool_next = min(pool_end, pool_next + (long long)__popc(need));
+          need = __ballot_sync(full, !alive);
+          continue;
+        }
+        long long p = 0;
+        if (lane == 0) p = (long long)atomicAdd(a.next, (unsigned long long)pool);
+        p = __shfl_sync(full, p, 0);
+        if (p >= total) exhausted = true;
+        else { pool_next = p; pool_end = min(p + pool, total); }
+      }
+      if (need == full) break;   // every lane idle, and the pools are exhausted
+    }
+    // every live lane's next steps, without a look at the others between them
+    for (int k = 0; k < refill.steps && alive; ++k)
+    {
+      bool retire = it >= a.iterations;
+      if constexpr (SCHEME == flow_frozen)
+      {
+        if (!retire)
+        {
+          float3 v;
+          if (!sample_inside_cached(a.f, cache, pos, v) || is_zero(v)) retire = true;
+          else { pos = frozen_step(a.rule, pos, v, hist); ++steps; ++it; }
+        }
+      }
+      else
+      {
+        if (!retire) retire = !local_inside(a.f, q);
+        if (!retire)
+        {
+          const float3 v = sample_local(a.f, cache, q.ix, q.iy, q.iz, q.ux, q.uy, q.uz);
+          if (is_zero_local(a.f, v)) retire = true;
+          else { flow_step<SCHEME>(a, cache, q, v, hist); ++steps; ++it; }
+        }
+      }
+      if (retire) { alive = false; ended = true; }
+    }
+  }
+  const unsigned int warp_steps = __reduce_add_sync(full, steps);
+  if (lane == 0 && warp_steps) atomicAdd(a.steps, (unsigned long long)warp_steps);
+}
+
+const void* flow_map_kernels[flow_schemes] = {
+  (const void*)flow_map_kernel<flow_frozen>, (const void*)flow_map_kernel<flow_classic>, (const void*)flow_map_kernel<flow_midpoint>,
+  (const void*)flow_map_kernel<flow_cash_karp>, (const void*)flow_map_kernel<flow_dormand_prince>,
+  (const void*)flow_map_kernel<flow_fehlberg>, (const void*)flow_map_kernel<flow_adams_bashforth>,
+  (const void*)flow_map_kernel<flow_adams_moulton>};
+
+// Resident CTAs of the kernel on the device, all SMs together.
+cudaError_t flow_map_resident(flow_scheme scheme, int device, int* ctas)
+{
+  int per_sm = 0, sms = 0;
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flow_map_kernels[scheme], 128, 0);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  *ctas = std::max(1, per_sm) * std::max(1, sms);
+  return e;
+}
+
+// `total` > 0 seeds on at most `resident` CTAs; pools as batch_pool_for cuts
+// them (256 seeds where every warp gets several pools, 32 where few do).
+cudaError_t launch_flow_map_kernel(const flow_map_args& a, flow_scheme scheme, int resident, cudaStream_t stream)
 {
   const long long total = (long long)a.px * a.py * a.pz;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned int steps = 0;
-  if (i < total)
-  {
-    const int iz = int(i % a.pz);
-    const int iy = int((i / a.pz) % a.py);
-    const int ix = int(i / ((long long)a.pz * a.py));
-    float4 pos = make_float4(__fadd_rn(a.ox, __fmul_rn(a.sx, float(ix))), __fadd_rn(a.oy, __fmul_rn(a.sy, float(iy))),
-                             __fadd_rn(a.oz, __fmul_rn(a.sz, float(iz))), 0.0f);
-    corner_cache cache;
-    frozen_history hist;
-    if constexpr (FROZEN)
-    {
-      for (int it = 1; it < a.iterations; ++it)
-      {
-        float3 v;
-        if (!sample_inside_cached(a.f, cache, pos, v) || is_zero(v)) break;
-        pos = frozen_step(a.rule, pos, v, hist);
-        ++steps;
-      }
-    }
-    else
-    {
-      // Re-sampled schemes in local cell coordinates (cell + offset +
-      // compensation); the position leaves them once, at the end.
-      local_position q = to_local(a.f, pos);
-      for (int it = 1; it < a.iterations; ++it)
-      {
-        if (!local_inside(a.f, q)) break;
-        const float3 v = sample_local(a.f, cache, q.ix, q.iy, q.iz, q.ux, q.uy, q.uz);
-        if (is_zero_local(a.f, v)) break;
-        general_step_local(a.f, cache, a.rule, q, v, hist);
-        ++steps;
-      }
-      if (steps) pos = flow_position(a.f, q);
-    }
-    // With iterations <= 1 the reference never assigns the voxel; it keeps the
-    // seed position here.
-    if (ix < a.fx && iy < a.fy && iz < a.fz)
-      a.flow[((long long)ix * a.fy + iy) * a.fz + iz] = pos;
-  }
-  const unsigned int warp_steps = __reduce_add_sync(0xffffffffu, steps);
-  if ((threadIdx.x & 31) == 0 && warp_steps) atomicAdd(a.steps, (unsigned long long)warp_steps);
+  int pool = (int)std::min<long long>(256, std::max<long long>(32, total / (4LL * resident * 4) / 32 * 32));
+  const unsigned grid = (unsigned)std::min<long long>(resident, (total + 4 * pool - 1) / (4 * pool));
+  refill_rule refill = refill_for(total, resident * 128LL);
+  void* args[] = {(void*)&a, (void*)&pool, (void*)&refill};
+  return cudaLaunchKernel(flow_map_kernels[scheme], grid, 128, args, 0, stream);
 }
 
 // Eigenvalues of the symmetric 3x3 matrix a (in place on its diagonal) by
@@ -213,22 +328,28 @@ void launch_ftle_kernel(const ftle_args& a, unsigned grid, cudaStream_t stream)
 }
 }
 
-void launch_flow_map(pars_gpu_context& ctx, const field_view& f, const step_rule& rule, int iterations,
-                     const float offset[3], const float fm_spacing[3], const int seeds_per_dimension[3],
-                     const int fm_shape[3], float4* flow, unsigned long long* steps)
+const unsigned long long* launch_flow_map(pars_gpu_context& ctx, const field_view& f, const step_rule& rule, int iterations,
+                                          const float offset[3], const float fm_spacing[3], const int seeds_per_dimension[3],
+                                          const int fm_shape[3], float4* flow)
 {
+  ctx.counters.reserve(sizeof(unsigned long long) * 2);   // steps taken, seeds handed out
+  auto* counters = ctx.counters.as<unsigned long long>();
+  PARS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 2, ctx.stream));
   flow_map_args a;
   a.f = f; a.rule = rule; a.iterations = iterations;
   a.ox = offset[0]; a.oy = offset[1]; a.oz = offset[2];
   a.sx = fm_spacing[0]; a.sy = fm_spacing[1]; a.sz = fm_spacing[2];
   a.px = seeds_per_dimension[0]; a.py = seeds_per_dimension[1]; a.pz = seeds_per_dimension[2];
   a.fx = fm_shape[0]; a.fy = fm_shape[1]; a.fz = fm_shape[2];
-  a.flow = flow; a.steps = steps;
+  a.flow = flow; a.steps = counters; a.next = counters + 1;
   const long long total = (long long)a.px * a.py * a.pz;
-  if (total <= 0) return;
+  if (total <= 0) return counters;
+  const flow_scheme scheme = flow_scheme_of(rule);
+  int& resident = ctx.flow_map_ctas[scheme];
+  if (resident < 0) PARS_CUDA(flow_map_resident(scheme, ctx.device, &resident));
   launch_scope scope(ctx, "advect_flow_map");
-  if (rule.frozen) flow_map_kernel<true><<<(unsigned)((total + 127) / 128), 128, 0, ctx.stream>>>(a);
-  else             flow_map_kernel<false><<<(unsigned)((total + 127) / 128), 128, 0, ctx.stream>>>(a);
+  PARS_CUDA(launch_flow_map_kernel(a, scheme, resident, ctx.stream));
+  return counters;
 }
 
 void launch_ftle(pars_gpu_context& ctx, const field_view& flow, double time, int mode, float* out)
@@ -274,13 +395,15 @@ __global__ void steps_to_int64_kernel(const unsigned long long* __restrict__ cou
 }
 
 // Host code must not use the array's name as a device address: it is a host
-// stand-in.  The device address is looked up once per device, with that device
-// current, and cached; later calls on the device reuse it.
+// stand-in.  The device address, and how many CTAs of the flow-map kernel fit
+// on the device, are looked up once per device, with that device current, and
+// cached; later calls on the device reuse them.
 constexpr int no_alloc_max_devices = 64;
 std::mutex no_alloc_mutex;
 float4* no_alloc_address[no_alloc_max_devices] = {};
+int no_alloc_resident[no_alloc_max_devices][flow_schemes] = {};
 
-int32_t no_alloc_scratch_address(int device, float4** out)
+int32_t no_alloc_device(int device, flow_scheme scheme, float4** out, int* resident)
 {
   if (device < 0 || device >= no_alloc_max_devices) return PARS_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> lock(no_alloc_mutex);
@@ -288,9 +411,17 @@ int32_t no_alloc_scratch_address(int device, float4** out)
   {
     void* p = nullptr;
     if (cudaGetSymbolAddress(&p, no_alloc_scratch) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
+    // every scheme's at once: a later call may be the first of its scheme inside a stream capture
+    for (int k = 0; k < flow_schemes; ++k)
+      if (flow_map_resident(flow_scheme(k), device, &no_alloc_resident[device][k]) != cudaSuccess)
+      {
+        (void)cudaGetLastError();
+        return PARS_ERR_CUDA;
+      }
     no_alloc_address[device] = static_cast<float4*>(p);
   }
   *out = no_alloc_address[device];
+  *resident = no_alloc_resident[device][scheme];
   return PARS_OK;
 }
 }
@@ -346,7 +477,9 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
   float4* scratch = nullptr;
-  const int32_t status = no_alloc_scratch_address(device, &scratch);
+  const flow_scheme scheme = flow_scheme_of(rule);
+  int resident = 0;
+  const int32_t status = no_alloc_device(device, scheme, &scratch, &resident);
   if (status != PARS_OK) return status;
   float4* field_data = scratch;
   float4* flow = scratch + no_alloc_max_voxels;
@@ -361,8 +494,8 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   f.maxx = offset[0] + size[0]; f.maxy = offset[1] + size[1]; f.maxz = offset[2] + size[2];
   set_reciprocals(f);
 
-  // The counter keeps the previous call's value: clear it first.
-  if (cudaMemsetAsync(counter, 0, sizeof(unsigned long long), s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
+  // The counters (steps, seeds handed out) keep the previous call's values: clear them first.
+  if (cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
   pack_into_scratch_kernel<<<(unsigned)((voxels + 255) / 256), 256, 0, s>>>(device_xyz, field_data, voxels);
   if (cudaGetLastError() != cudaSuccess) return PARS_ERR_CUDA;
 
@@ -372,11 +505,8 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   a.sx = spacing[0]; a.sy = spacing[1]; a.sz = spacing[2];
   a.px = seeds[0]; a.py = seeds[1]; a.pz = seeds[2];
   a.fx = shape[0]; a.fy = shape[1]; a.fz = shape[2];
-  a.flow = flow; a.steps = counter;
-  const long long total = (long long)a.px * a.py * a.pz;
-  if (rule.frozen) flow_map_kernel<true><<<(unsigned)((total + 127) / 128), 128, 0, s>>>(a);
-  else             flow_map_kernel<false><<<(unsigned)((total + 127) / 128), 128, 0, s>>>(a);
-  if (cudaGetLastError() != cudaSuccess) return PARS_ERR_CUDA;
+  a.flow = flow; a.steps = counter; a.next = counter + 1;
+  if (launch_flow_map_kernel(a, scheme, resident, s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
 
   ftle_args t;
   t.flow = flow; t.nx = shape[0]; t.ny = shape[1]; t.nz = shape[2];

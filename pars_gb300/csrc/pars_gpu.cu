@@ -1922,16 +1922,14 @@ int32_t pars_gpu_flow_map_generate(pars_gpu_context* ctx, int32_t field, int32_t
       throw error(PARS_ERR_UNSUPPORTED, "unsteady flow maps integrate with RK4 or Euler");
     if (rule.frozen || iterations <= 1 || rule.scheme != scheme_classic)
     {
-      // One seed per thread: the reference's scheme bit for bit (one field
+      // The flow-map kernel: the reference's scheme bit for bit (one field
       // sample per step: at 64 registers this kernel keeps more warps
       // resident than the batched engine's frozen class, 57 against 53 G
       // steps/s on the 256^3 flow map), the iterations <= 1 case, where every
       // voxel keeps its seed position, and the re-sampled stages of the
       // general schemes.
-      ctx->counters.reserve(sizeof(unsigned long long) * 2);
-      auto* counter = ctx->counters.as<unsigned long long>();
-      PARS_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned long long), ctx->stream));
-      launch_flow_map(*ctx, f.view(), rule, iterations, f.offset, entry->spacing, seeds, entry->shape, entry->data.as<float4>(), counter);
+      const unsigned long long* counter = launch_flow_map(*ctx, f.view(), rule, iterations, f.offset, entry->spacing, seeds, entry->shape,
+                                                          entry->data.as<float4>());
       if (steps)
       {
         unsigned long long s = 0;

@@ -362,16 +362,13 @@ bool engine_job(const batch_job_device& j) { return j.rule.frozen || j.rule.sche
 // The per-seed flow-map kernel for one request; returns its steps.
 long long per_seed_flow_map(pars_gpu_context& c, const ftle_work& w)
 {
-  device_buffer counter;
-  counter.reserve(sizeof(unsigned long long));
-  PARS_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(unsigned long long), c.stream));
   const batch_job_device& j = w.job;
   const float offset[3] = {j.ox, j.oy, j.oz}, spacing[3] = {j.sx, j.sy, j.sz};
   const int seeds[3] = {j.px, j.py, j.pz}, shape[3] = {j.ux, j.uy, j.uz};
-  launch_flow_map(c, j.field, j.rule, w.r->s.seed_generation_iterations, offset, spacing, seeds, shape,
-                  w.flow.as<float4>(), counter.as<unsigned long long>());
+  const unsigned long long* counter = launch_flow_map(c, j.field, j.rule, w.r->s.seed_generation_iterations, offset, spacing, seeds,
+                                                      shape, w.flow.as<float4>());
   unsigned long long steps = 0;
-  PARS_CUDA(cudaMemcpyAsync(&steps, counter.get(), sizeof(steps), cudaMemcpyDeviceToHost, c.stream));
+  PARS_CUDA(cudaMemcpyAsync(&steps, counter, sizeof(steps), cudaMemcpyDeviceToHost, c.stream));
   PARS_CUDA(cudaStreamSynchronize(c.stream));
   return (long long)steps;
 }
