@@ -3,9 +3,10 @@
 //
 // The grid holds as many CTAs as fit on the GPU at once.  Work is a queue of
 // pools (`pool` consecutive seeds of one job); a warp takes pools with one
-// atomic and hands their seeds to its lanes.  A lane whose particle retires
-// takes the next seed of the pool at once (warp ballot + prefix), so lanes do
-// not idle while the rest of the warp finishes long particles.  All lanes of a
+// atomic and hands their seeds to its lanes.  Lanes whose particles have
+// retired take the next seeds of the pool (refill_rule, warp ballot +
+// prefix), so lanes do not idle while the rest of the warp finishes long
+// particles.  All lanes of a
 // warp work on the same job; a warp moves to another job only when its lanes
 // have drained, so job parameters stay warp-uniform.
 //
@@ -76,13 +77,37 @@ template <int CLASS>
 struct lane_cache { corner_cache k; };
 template <> struct lane_cache<batch_unsteady> { corner_cache2 k; };
 
+
+// An ended particle's outputs: its last position and its step count.
+template <int CLASS>
+__device__ __forceinline__ void write_end(const batch_job_device& J, const field_view& f, long long seed, int steps, float4 pos,
+                                          const local_position& local)
+{
+  if (J.end_positions)
+  {
+    long long out = seed;
+    bool write = true;
+    if (!J.seeds && J.ux > 0)
+    {
+      // lattice seed -> output voxel of the flow map's own shape
+      int ix, iy, iz;
+      lattice_index(seed, J.py, J.pz, ix, iy, iz);
+      write = ix < J.ux && iy < J.uy && iz < J.uz;
+      out = ((long long)ix * J.uy + iy) * J.uz + iz;
+    }
+    if constexpr (CLASS != batch_frozen) pos = flow_position(f, local);
+    if (write) J.end_positions[out] = pos;
+  }
+  if (J.end_steps) J.end_steps[seed] = steps;
+}
+
 // CLASS batch_steady: re-sampled stages, every job on a steady field (one
 // slice).  batch_unsteady: re-sampled stages, jobs may have several time
 // slices (a steady job works too).  batch_frozen: the frozen scheme.
 template <int THREADS, int MIN_BLOCKS, int CLASS, bool HORIZON = false>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS)
 batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long long total_pools,
-                    unsigned long long* __restrict__ pool_counter, const __grid_constant__ batch_horizon_args hz)
+                    unsigned long long* __restrict__ pool_counter, refill_rule refill, const __grid_constant__ batch_horizon_args hz)
 {
   const int lane = threadIdx.x & 31;
   const unsigned lanes_below = (1u << lane) - 1u;
@@ -93,7 +118,7 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
   bool exhausted = false;
   unsigned int job_steps = 0;       // this lane's steps on the current job
   // lane state
-  bool alive = false;
+  bool alive = false, ended = false;              // ended: holds a particle not yet written
   long long seed = 0;
   int steps = 0;
   float4 pos = make_float4(0.f, 0.f, 0.f, 0.f);   // seed / end position
@@ -108,7 +133,7 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
   slice_clock clock {};
   const step_rule* rule = nullptr;   // frozen jobs: the coefficients, read where they lie
   // horizon launches: steps this warp has taken
-  int iteration = 0;
+  int iteration = 0, next_look = 16;
 
   if constexpr (HORIZON)
   {
@@ -146,68 +171,71 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
 
   for (;;)
   {
-    // ---- refill idle lanes ---------------------------------------------------
+    // ---- write ended particles, refill idle lanes -----------------------------
     unsigned need = __ballot_sync(full_mask, !alive);
-    while (need)
+    if (__popc(need) >= (exhausted || pending >= 0 ? 32 : refill.lanes))
     {
-      if (pool_next < pool_end)
+      if (ended) { write_end<CLASS>(jobs[job], f, seed, steps, pos, local); ended = false; }
+      while (need)
       {
-        const long long s = pool_next + __popc(need & lanes_below);
-        if (!alive && s < pool_end)
+        if (pool_next < pool_end)
         {
-          const batch_job_device& J = jobs[job];
-          seed = s;
-          if (J.seeds) pos = J.seeds[s];
-          else
+          const long long s = pool_next + __popc(need & lanes_below);
+          if (!alive && s < pool_end)
           {
-            const int iz = int(s % J.pz);
-            const int iy = int((s / J.pz) % J.py);
-            const int ix = int(s / ((long long)J.pz * J.py));
-            pos = make_float4(__fadd_rn(J.ox, __fmul_rn(J.sx, float(ix))), __fadd_rn(J.oy, __fmul_rn(J.sy, float(iy))),
-                              __fadd_rn(J.oz, __fmul_rn(J.sz, float(iz))), 0.0f);
+            const batch_job_device& J = jobs[job];
+            seed = s;
+            if (J.seeds) pos = J.seeds[s];
+            else
+            {
+              int ix, iy, iz;
+              lattice_index(s, J.py, J.pz, ix, iy, iz);
+              pos = make_float4(__fadd_rn(J.ox, __fmul_rn(J.sx, float(ix))), __fadd_rn(J.oy, __fmul_rn(J.sy, float(iy))),
+                                __fadd_rn(J.oz, __fmul_rn(J.sz, float(iz))), 0.0f);
+            }
+            if constexpr (CLASS == batch_frozen) hist = frozen_history();
+            else local = to_local(f, pos);
+            steps = 0;
+            alive = true;
           }
-          if constexpr (CLASS == batch_frozen) hist = frozen_history();
-          else local = to_local(f, pos);
-          steps = 0;
-          alive = true;
+          pool_next = min(pool_end, pool_next + (long long)__popc(need));
+          need = __ballot_sync(full_mask, !alive);
+          continue;
         }
-        pool_next = min(pool_end, pool_next + (long long)__popc(need));
-        need = __ballot_sync(full_mask, !alive);
-        continue;
-      }
-      if (exhausted) break;
-      long long p = pending;
-      if (p < 0)
-      {
-        if (lane == 0) p = (long long)atomicAdd(pool_counter, 1ULL);
-        p = __shfl_sync(full_mask, p, 0);
-      }
-      if (p >= total_pools) { exhausted = true; break; }
-      const int pj = find_job(jobs, njobs, p);
-      if (pj != job)
-      {
-        if (__any_sync(full_mask, alive)) { pending = p; break; }   // drain the current job first
-        // switch job: flush this lane's step count, load the new parameters
-        if (job >= 0)
+        if (exhausted) break;
+        long long p = pending;
+        if (p < 0)
         {
-          const unsigned int total = __reduce_add_sync(full_mask, job_steps);
-          if (lane == 0 && total) atomicAdd(jobs[job].steps, (unsigned long long)total);
+          if (lane == 0) p = (long long)atomicAdd(pool_counter, 1ULL);
+          p = __shfl_sync(full_mask, p, 0);
         }
-        job_steps = 0;
-        job = pj;
-        const batch_job_device& J = jobs[job];
-        f = J.field; ta = J.time; h = J.rule.h; rk4 = J.rule.rk4; max_steps = J.max_steps; clock = J.clock;
-        rule = &J.rule;
-        cache = lane_cache<CLASS>();
+        if (p >= total_pools) { exhausted = true; break; }
+        const int pj = find_job(jobs, njobs, p);
+        if (pj != job)
+        {
+          if (__any_sync(full_mask, alive)) { pending = p; break; }   // drain the current job first
+          // switch job: flush this lane's step count, load the new parameters
+          if (job >= 0)
+          {
+            const unsigned int total = __reduce_add_sync(full_mask, job_steps);
+            if (lane == 0 && total) atomicAdd(jobs[job].steps, (unsigned long long)total);
+          }
+          job_steps = 0;
+          job = pj;
+          const batch_job_device& J = jobs[job];
+          f = J.field; ta = J.time; h = J.rule.h; rk4 = J.rule.rk4; max_steps = J.max_steps; clock = J.clock;
+          rule = &J.rule;
+          cache = lane_cache<CLASS>();
+        }
+        pending = -1;
+        pool_next = (p - jobs[job].first_pool) * jobs[job].pool;
+        pool_end = min(pool_next + jobs[job].pool, jobs[job].seed_count);
       }
-      pending = -1;
-      pool_next = (p - jobs[job].first_pool) * jobs[job].pool;
-      pool_end = min(pool_next + jobs[job].pool, jobs[job].seed_count);
-    }
-    if (!__any_sync(full_mask, alive))
-    {
-      if (exhausted) break;
-      continue;   // switch to the pending job
+      if (need == full_mask)
+      {
+        if (exhausted) break;
+        continue;   // switch to the pending job
+      }
     }
 
     if constexpr (HORIZON)
@@ -215,17 +243,18 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
       // The first warp to reach the horizon raises the launch's stop flag;
       // the others see it within 16 steps, so the launch ends with every SM
       // busy to the end instead of waiting for its slowest warp.
-      ++iteration;
-      bool stop = iteration > hz.iterations;
-      if (!stop && (iteration & 15) == 0)
+      bool stop = iteration >= hz.iterations;
+      if (!stop && iteration >= next_look)
       {
         unsigned int flag = 0;
         if (lane == 0) flag = load_relaxed(hz.stop);
         stop = __shfl_sync(full_mask, flag, 0) != 0u;
+        next_look = iteration + 16;
       }
       if (stop)
       {
-        if (lane == 0 && iteration > hz.iterations) store_relaxed(hz.stop, 1u);
+        if (lane == 0 && iteration >= hz.iterations) store_relaxed(hz.stop, 1u);
+        if (ended) write_end<CLASS>(jobs[job], f, seed, steps, pos, local);
         // park: the group record, then the live lanes' particles in lane order
         const unsigned live = __ballot_sync(full_mask, alive);
         unsigned int g = 0;
@@ -255,8 +284,14 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
       }
     }
 
-    // ---- one step of every live lane -------------------------------------------
-    if (alive)
+    // ---- the next steps of every live lane, without a look at the others --------
+    int ahead = refill.steps;
+    if constexpr (HORIZON)
+    {
+      ahead = min(ahead, hz.iterations - iteration);
+      iteration += ahead;
+    }
+    for (int k = 0; k < ahead && alive; ++k)
     {
       bool retire = steps >= max_steps;
       if constexpr (CLASS == batch_frozen)
@@ -281,7 +316,6 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
           if (is_zero_local(f, k1)) retire = true;
           else { local_unsteady_step(f, ta, clock, cache.k, rk4, h, local, k1, t); ++steps; ++job_steps; }
         }
-        if (retire) pos = flow_position(f, local);
       }
       else
       {
@@ -293,27 +327,8 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
           if (is_zero_local(f, k1)) retire = true;
           else { local_step(f, cache.k, rk4, h, local, k1); ++steps; ++job_steps; }
         }
-        if (retire) pos = flow_position(f, local);
       }
-      if (retire)
-      {
-        const batch_job_device& J = jobs[job];
-        if (J.end_positions)
-        {
-          long long out = seed;
-          bool write = true;
-          if (!J.seeds && J.ux > 0)
-          {
-            // lattice seed -> output voxel of the flow map's own shape
-            const int iz = int(seed % J.pz), iy = int((seed / J.pz) % J.py), ix = int(seed / ((long long)J.pz * J.py));
-            write = ix < J.ux && iy < J.uy && iz < J.uz;
-            out = ((long long)ix * J.uy + iy) * J.uz + iz;
-          }
-          if (write) J.end_positions[out] = pos;
-        }
-        if (J.end_steps) J.end_steps[seed] = steps;
-        alive = false;
-      }
+      if (retire) { alive = false; ended = true; }
     }
   }
   if (job >= 0)
@@ -364,7 +379,7 @@ int batch_pool_for(pars_gpu_context& ctx, int job_class, int v, long long seeds)
 }
 
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int v, const batch_job_device* jobs, int njobs,
-                         long long total_pools, unsigned long long* counter)
+                         long long total_pools, long long seeds, unsigned long long* counter)
 {
   if (total_pools <= 0) return;
   const variant& var = variants[job_class][v];
@@ -375,8 +390,9 @@ void launch_batch_advect(pars_gpu_context& ctx, int job_class, int v, const batc
   const long long warps_needed = total_pools;   // at least one pool per warp
   const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(persistent, (warps_needed * 32 + var.threads - 1) / var.threads));
   const batch_horizon_args none {};
+  refill_rule refill = refill_for(seeds, persistent * var.threads);
   launch_scope scope(ctx, "batch_advect");
-  void* args[] = {(void*)&jobs, (void*)&njobs, (void*)&total_pools, (void*)&counter, (void*)&none};
+  void* args[] = {(void*)&jobs, (void*)&njobs, (void*)&total_pools, (void*)&counter, (void*)&refill, (void*)&none};
   PARS_CUDA(cudaLaunchKernel(var.kernel, grid, var.threads, args, 0, ctx.stream));
 }
 
@@ -398,8 +414,10 @@ void launch_batch_advect_horizon(pars_gpu_context& ctx, int job_class, int v, co
   const unsigned grid = (unsigned)((want * 32 + var.threads - 1) / var.threads);
   // every parked group needs a warp of its own to resume it
   PARS_REQUIRE((long long)grid * (var.threads / 32) >= hz.in_count, "more parked groups than warps");
+  // more jobs may follow, and no warp may run past the horizon's stop flag for long
+  refill_rule refill {4, 8};
   launch_scope scope(ctx, "batch_advect_horizon");
-  void* args[] = {(void*)&jobs, (void*)&njobs, (void*)&total_pools, (void*)&counter, (void*)&hz};
+  void* args[] = {(void*)&jobs, (void*)&njobs, (void*)&total_pools, (void*)&counter, (void*)&refill, (void*)&hz};
   PARS_CUDA(cudaLaunchKernel(var.horizon_kernel, grid, var.threads, args, 0, ctx.stream));
 }
 }

@@ -459,7 +459,7 @@ int  batch_variant_threads(int variant);
 int  batch_pool_for(pars_gpu_context& ctx, int job_class, int variant, long long seeds);
 // job_class: batch_steady, batch_unsteady or batch_frozen.
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int variant, const batch_job_device* jobs, int njobs,
-                         long long total_chunks, unsigned long long* counter);
+                         long long total_pools, long long seeds, unsigned long long* counter);
 
 // Horizon launches of the batched engine.  A warp that has taken `iterations`
 // steps, or that sees another warp's stop flag, parks as one group: its job (an index into the launch's job table),

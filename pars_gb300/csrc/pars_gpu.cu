@@ -865,7 +865,7 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
       PARS_CUDA(cudaMemcpyAsync(device_jobs, jobs.data(), sizeof(batch_job_device) * count, cudaMemcpyHostToDevice, ctx.stream));
       PARS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (count + 1), ctx.stream));
       PARS_CUDA(cudaEventRecord(a, ctx.stream));
-      launch_batch_advect(ctx, c, v, device_jobs, count, pools, counters);
+      launch_batch_advect(ctx, c, v, device_jobs, count, pools, seeds, counters);
       PARS_CUDA(cudaEventRecord(b, ctx.stream));
       PARS_CUDA(cudaEventSynchronize(b));
       float ms = 0.0f;
@@ -936,24 +936,24 @@ std::vector<unsigned long long> execute_batch(pars_gpu_context& ctx, std::vector
   ctx.batch_counters.reserve(sizeof(unsigned long long) * (count + C));
   auto* counters = ctx.batch_counters.as<unsigned long long>();
   auto* device_jobs = ctx.batch_jobs.as<batch_job_device>();
-  long long pools[C] = {};
+  long long pools[C] = {}, seeds[C] = {};
   for (int c = 0; c < C; ++c)
   {
     if (size[c] == 0) continue;
-    long long seeds = 0;
     for (int k = first[c]; k < first[c] + size[c]; ++k)
     {
       queue[k].steps = counters + C + k;
-      seeds += queue[k].seed_count;
+      seeds[c] += queue[k].seed_count;
     }
     const int shape = variant >= 0 ? variant : ctx.batch_variant[c];
-    pools[c] = number_pools(queue.data() + first[c], size[c], batch_pool_for(ctx, c, shape, seeds));
+    pools[c] = number_pools(queue.data() + first[c], size[c], batch_pool_for(ctx, c, shape, seeds[c]));
   }
   PARS_CUDA(cudaMemcpyAsync(device_jobs, queue.data(), sizeof(batch_job_device) * count, cudaMemcpyHostToDevice, ctx.stream));
   PARS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (count + C), ctx.stream));
   for (int c = 0; c < C; ++c)
     if (size[c] > 0)
-      launch_batch_advect(ctx, c, variant >= 0 ? variant : ctx.batch_variant[c], device_jobs + first[c], size[c], pools[c], counters + c);
+      launch_batch_advect(ctx, c, variant >= 0 ? variant : ctx.batch_variant[c], device_jobs + first[c], size[c], pools[c], seeds[c],
+                          counters + c);
   std::vector<unsigned long long> steps(count + C);
   PARS_CUDA(cudaMemcpyAsync(steps.data(), counters, sizeof(unsigned long long) * (count + C), cudaMemcpyDeviceToHost, ctx.stream));
   PARS_CUDA(cudaStreamSynchronize(ctx.stream));
