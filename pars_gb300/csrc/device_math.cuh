@@ -743,26 +743,12 @@ __device__ __forceinline__ float4 to_absolute(const field_view& f, const local_p
 // carries each coordinate to about 34 bits.  Frozen-scheme flow maps, the
 // reference's FP32 state, store w = 0 (no residual).
 
-// ulp of a normal FP32 x with |x| >= 2^-103; 0 for smaller x (no residual).
-__device__ __forceinline__ float residual_ulp(float x)
-{
-  const unsigned e = __float_as_uint(x) & 0x7f800000u;
-  return e > (23u << 23) ? __uint_as_float(e - (23u << 23)) : 0.0f;
-}
-
 // 1 / ulp(x) for a normal x with |x| >= 2^-103 (a power of two, so scaling
 // by it is exact).
 __device__ __forceinline__ float residual_inverse_ulp(float x)
 {
   const unsigned e = __float_as_uint(x) & 0x7f800000u;
   return __uint_as_float((277u << 23) - e);
-}
-
-// The residual of x coded in w's bits [shift, shift + 10).
-__device__ __forceinline__ float residual_value(float x, unsigned w, int shift)
-{
-  const int q = int(w << (22 - shift)) >> 22;
-  return float(q) * (residual_ulp(x) * (1.0f / 1022.0f));
 }
 
 // One coordinate o + (i + u + l) h of a local position as its correctly
