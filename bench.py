@@ -328,7 +328,8 @@ def run_render(args):
             rgba = image()
         wall = (time.perf_counter() - t0) / args.steps
         build_ms, _ = ctx.profile_get("bvh_build")
-        render_ms, _ = ctx.profile_get("render")
+        # capsules drawn onto the screen, or a walk through the tree, then shading
+        render_ms = sum(ctx.profile_get(k)[0] for k in ("raster_count", "raster_begin", "raster", "tree_hits", "render"))
         ctx.profile_enable(False)
         batches = ctx.curves(s["batches"], vertices=True, colors=True, indices=True)
         host = [(b["vertices"], b["colors"], b["indices"]) for b in batches]

@@ -157,6 +157,7 @@ struct render_state
   long long     prims = 0;
   long long     leaves = 0;                     // BVH leaves (runs of 1 or 2 consecutive segments)
   const float4* vertices = nullptr;
+  long long     vertex_limit = 0;               // vertices there (every segment starts below it)
   const float4* colors = nullptr;               // nullptr: white
   float         radius = 1.0f;
   long long     curves_generation = -1;         // >= 0: the context's curves at that generation
@@ -177,11 +178,13 @@ struct render_state
   bool          camera_set = false;
   float         position[3] = {0, 0, 0}, corner[3] = {0, 0, 0}, du[3] = {0, 0, 0}, dv[3] = {0, 0, 0};
   float         forward[3] = {0, 0, 1}, up[3] = {0, 1, 0};
+  float         right[3] = {0, 0, 0}, above[3] = {0, 0, 0}, ahead[3] = {0, 0, 0}, focal = 0;   // orthonormal basis, pixels per slope
   int           width = 0, height = 0;
   // accumulated frames
   bool          accum_valid = false;
   long long     frames = 0;
   device_buffer accum, jitter, status, image, thresholds;
+  device_buffer directions, pixel_keys, raster_count, raster_slices;   // capsules onto the screen: rays, closest hits, pixels covered
   float         srgb_thresholds[255];
 };
 
@@ -397,6 +400,8 @@ void exclusive_sum(pars_gpu_context& ctx, const int* in, long long* out, long lo
 // Stable sort of (key, value) pairs by the low `bits` bits of the key.
 void sort_pairs(pars_gpu_context& ctx, const unsigned long long* keys_in, unsigned long long* keys_out,
                 const unsigned int* values_in, unsigned int* values_out, long long count, int bits);
+void sort_pairs(pars_gpu_context& ctx, const unsigned int* keys_in, unsigned int* keys_out, const unsigned int* values_in,
+                unsigned int* values_out, long long count, int bits);
 // Gathers the sorted exit queue into the next round's particle list and
 // accumulates per-block maximum remaining_iterations and particle counts.
 void launch_gather_exits(pars_gpu_context& ctx, const pars_particle* exits, const unsigned int* order,
@@ -533,14 +538,14 @@ void launch_ftle(pars_gpu_context& ctx, const field_view& flow, double time, int
 
 // Ray tracer (render_kernels.cu).
 void render_jitter(long long frame, float& jx, float& jy);
-void render_camera(const float position[3], const float forward[3], const float up[3], int width, int height,
-                   float corner[3], float du[3], float dv[3]);
+void render_camera(render_state& r);
 void render_clear(render_state& r);
 void render_use_context_curves(pars_gpu_context& ctx, render_state& r);
 // Prims of curve spans inside caller-owned buffers: each span is (start vertex
 // of its batch in `vertices`, first index in `indices`, index count).
-void render_use_spans(pars_gpu_context& ctx, render_state& r, const float4* vertices, const float4* colors, const int* indices,
-                      const std::vector<std::array<long long, 3>>& spans);
+// vertex_count: vertices in the buffer.
+void render_use_spans(pars_gpu_context& ctx, render_state& r, const float4* vertices, long long vertex_count, const float4* colors,
+                      const int* indices, const std::vector<std::array<long long, 3>>& spans);
 // Camera and image size (ray_tracer.cpp:213-229); clears the accumulation.
 void render_set_view(render_state& r, const float position[3], const float forward[3], const float up[3], int width, int height);
 void render_build(pars_gpu_context& ctx, render_state& r);

@@ -531,7 +531,7 @@ void render_request(pars_gpu_service& svc, pars_gpu_context& c, request& r, cons
   render_state& rs = *c.render;
   std::vector<std::array<long long, 3>> spans;
   for (const auto& s : r.spans) spans.push_back({s.store_vertex_offset, s.store_index_offset, s.index_count});
-  render_use_spans(c, rs, store.vertices.as<const float4>(), store.colors.as<const float4>(), store.indices.as<const int>(), spans);
+  render_use_spans(c, rs, store.vertices.as<const float4>(), (long long)(store.vertices.bytes() / sizeof(float4)), store.colors.as<const float4>(), store.indices.as<const int>(), spans);
   const float radius = r.s.raytracing_streamline_radius;
   rs.radius = radius != 0.0f ? radius : 1.0f;                       // pipeline.cpp:306
   rs.has_volume = false;

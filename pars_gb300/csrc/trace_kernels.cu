@@ -745,8 +745,11 @@ void exclusive_sum(pars_gpu_context& ctx, const int* in, long long* out, long lo
   PARS_CUDA(cub::DeviceScan::ExclusiveSum(ctx.cub_temp.get(), bytes, wide, out, count + 1, ctx.stream));
 }
 
-void sort_pairs(pars_gpu_context& ctx, const unsigned long long* keys_in, unsigned long long* keys_out,
-                const unsigned int* values_in, unsigned int* values_out, long long count, int bits)
+namespace
+{
+template <typename key_type>
+void radix_sort_pairs(pars_gpu_context& ctx, const key_type* keys_in, key_type* keys_out, const unsigned int* values_in,
+                      unsigned int* values_out, long long count, int bits)
 {
   if (count <= 0) return;
   std::size_t bytes = 0;
@@ -754,6 +757,19 @@ void sort_pairs(pars_gpu_context& ctx, const unsigned long long* keys_in, unsign
   ctx.cub_temp.reserve(bytes);
   launch_scope scope(ctx, "exit_sort");
   PARS_CUDA(cub::DeviceRadixSort::SortPairs(ctx.cub_temp.get(), bytes, keys_in, keys_out, values_in, values_out, count, 0, bits, ctx.stream));
+}
+}
+
+void sort_pairs(pars_gpu_context& ctx, const unsigned long long* keys_in, unsigned long long* keys_out,
+                const unsigned int* values_in, unsigned int* values_out, long long count, int bits)
+{
+  radix_sort_pairs(ctx, keys_in, keys_out, values_in, values_out, count, bits);
+}
+
+void sort_pairs(pars_gpu_context& ctx, const unsigned int* keys_in, unsigned int* keys_out, const unsigned int* values_in,
+                unsigned int* values_out, long long count, int bits)
+{
+  radix_sort_pairs(ctx, keys_in, keys_out, values_in, values_out, count, bits);
 }
 
 void launch_gather_exits(pars_gpu_context& ctx, const pars_particle* exits, const unsigned int* order,
