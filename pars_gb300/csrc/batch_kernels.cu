@@ -2,7 +2,7 @@
 // different sizes) in ONE persistent launch that drains a device work queue.
 //
 // The grid holds as many CTAs as fit on the GPU at once.  Work is a queue of
-// pools (`pool` consecutive seeds of one job); a warp takes pools with one
+// pools (pool_seeds consecutive seeds of one job); a warp takes pools with one
 // atomic and hands their seeds to its lanes.  Lanes whose particles have
 // retired take the next seeds of the pool (refill_rule, warp ballot +
 // prefix), so lanes do not idle while the rest of the warp finishes long
@@ -38,14 +38,13 @@ namespace pars
 namespace
 {
 constexpr unsigned full_mask = 0xffffffffu;
-// Seeds per pool.  Large pools keep a warp's lanes on neighbouring seeds, whose
-// particles share cache lines (256 is best where every warp gets many pools);
-// a job with fewer than pools_per_warp pools of that size per resident warp is
-// cut finer, down to one seed per lane, so that its seeds spread over every SM.
-// With 256 throughout, six pathline jobs of 4 k - 120 k seeds (1100 pools for
-// 1824 resident warps) took 7.79 ms, now 2.54 ms; served FTLE launches of up to
-// 500 k voxels 12.0 -> 4.9 ms; the 256^3 flow map keeps 256 (57.9 ms).
-constexpr int pool_largest = 256, pool_smallest = 32, pools_per_warp = 4;
+// Seeds per pool: one per lane.  Small pools spread a small launch over every SM
+// (six pathline jobs of 4 k - 120 k seeds: 2.5 ms, with 256 seeds a pool 7.8 ms),
+// and in a large one the warps of the whole GPU work on neighbouring seeds, whose
+// particles share cache lines (256^3 flow map with 32 / 64 / 128 / 256 / 512 seeds
+// a pool: 48.2 / 48.1 / 50.1 / 51.0 / 54 ms; pools as 3-D bricks of the lattice and
+// a range of pools per SM were slower, 51 - 55 ms).
+constexpr int pool_seeds = 32;
 
 __device__ __forceinline__ int find_job(const batch_job_device* __restrict__ jobs, int njobs, long long pool)
 {
@@ -228,8 +227,8 @@ batch_advect_kernel(const batch_job_device* __restrict__ jobs, int njobs, long l
           cache = lane_cache<CLASS>();
         }
         pending = -1;
-        pool_next = (p - jobs[job].first_pool) * jobs[job].pool;
-        pool_end = min(pool_next + jobs[job].pool, jobs[job].seed_count);
+        pool_next = (p - jobs[job].first_pool) * pool_seeds;
+        pool_end = min(pool_next + pool_seeds, jobs[job].seed_count);
       }
       if (need == full_mask)
       {
@@ -369,14 +368,7 @@ int batch_resident_warps(pars_gpu_context& ctx, int job_class, int v)
   return per_sm * var.threads / 32;
 }
 int batch_variant_threads(int v) { return variants[0][v].threads; }
-
-int batch_pool_for(pars_gpu_context& ctx, int job_class, int v, long long seeds)
-{
-  if (ctx.sm_count <= 0) PARS_CUDA(cudaDeviceGetAttribute(&ctx.sm_count, cudaDevAttrMultiProcessorCount, ctx.device));
-  const long long warps = (long long)std::max(1, batch_resident_warps(ctx, job_class, v)) * ctx.sm_count;
-  const long long pool = seeds / (warps * pools_per_warp) / pool_smallest * pool_smallest;
-  return (int)std::min<long long>(pool_largest, std::max<long long>(pool_smallest, pool));
-}
+int batch_pool_seeds() { return pool_seeds; }
 
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int v, const batch_job_device* jobs, int njobs,
                          long long total_pools, long long seeds, unsigned long long* counter)

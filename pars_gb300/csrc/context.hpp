@@ -103,7 +103,7 @@ struct field_entry
     v.ox = offset[0]; v.oy = offset[1]; v.oz = offset[2];
     v.hx = spacing[0]; v.hy = spacing[1]; v.hz = spacing[2];
     v.maxx = offset[0] + size[0]; v.maxy = offset[1] + size[1]; v.maxz = offset[2] + size[2];
-    set_reciprocals(v);
+    set_derived(v);
     return v;
   }
 };
@@ -450,7 +450,6 @@ struct batch_job_device
   int                 ux, uy, uz;     // lattice seeds: output voxel shape (0 = output per seed)
   float4*             end_positions;  // may be nullptr
   int*                end_steps;      // may be nullptr
-  int                 pool;           // seeds per pool (batch_pool_for)
   long long           first_pool;     // pools of all earlier jobs
   unsigned long long* steps;          // per-job step counter
 };
@@ -460,8 +459,7 @@ int  batch_variant_count();
 // Resident warps per SM of a job class's launch shape.
 int  batch_resident_warps(pars_gpu_context& ctx, int job_class, int variant);
 int  batch_variant_threads(int variant);
-// Seeds per pool for a launch (or a job) of `seeds` seeds.
-int  batch_pool_for(pars_gpu_context& ctx, int job_class, int variant, long long seeds);
+int  batch_pool_seeds();
 // job_class: batch_steady, batch_unsteady or batch_frozen.
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int variant, const batch_job_device* jobs, int njobs,
                          long long total_pools, long long seeds, unsigned long long* counter);

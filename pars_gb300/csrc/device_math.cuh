@@ -43,8 +43,8 @@ inline bool divides_fast(float hx, float hy, float hz)
   return in(hx) && in(hy) && in(hz);
 }
 
-// Reciprocals and the division flag of a view whose spacing is set.
-inline void set_reciprocals(field_view& f)
+// What follows from a view's shape and spacing.
+inline void set_derived(field_view& f)
 {
   f.inv_hx = 1.0f / f.hx; f.inv_hy = 1.0f / f.hy; f.inv_hz = 1.0f / f.hz;
   f.fast_division = divides_fast(f.hx, f.hy, f.hz) ? 1 : 0;
@@ -678,6 +678,33 @@ __device__ __forceinline__ bool in_unit_cube(float ux, float uy, float uz)
   return max(max(__float_as_uint(ux), __float_as_uint(uy)), __float_as_uint(uz)) < 0x3f800000u;
 }
 
+// i += floor(u), u -= floor(u).
+__device__ __forceinline__ void take_floor(int& i, float& u)
+{
+  const float fl = floorf(u);
+  i += int(fl);
+  u -= fl;
+}
+
+// The cell and weights of offset (wx, wy, wz) from cell (ix, iy, iz): the offset
+// moved into [0, 1)^3 and the cell accordingly, clamped to the grid (weight 0 or
+// 1).  One test covers the clamp, which only points that left the grid need
+// (three clamps at every cell change cost 2 % of a flow map).  (The floor by
+// rounding additions, at full rate, was slower: 20.4 against 19.8 ms for 192^3.
+// The additions compete with the blend, floorf and the conversion do not.)
+__device__ __forceinline__ void find_cell(const field_view& f, int& ix, int& iy, int& iz, float& wx, float& wy, float& wz)
+{
+  take_floor(ix, wx);
+  take_floor(iy, wy);
+  take_floor(iz, wz);
+  if (unsigned(ix) > unsigned(f.nx - 2) || unsigned(iy) > unsigned(f.ny - 2) || unsigned(iz) > unsigned(f.nz - 2))
+  {
+    if (ix < 0) { ix = 0; wx = 0.0f; } else if (ix > f.nx - 2) { ix = f.nx - 2; wx = 1.0f; }
+    if (iy < 0) { iy = 0; wy = 0.0f; } else if (iy > f.ny - 2) { iy = f.ny - 2; wy = 1.0f; }
+    if (iz < 0) { iz = 0; wz = 0.0f; } else if (iz > f.nz - 2) { iz = f.nz - 2; wz = 1.0f; }
+  }
+}
+
 // Velocity (cells per unit time) at cell (cx, cy, cz) + (ux, uy, uz), where
 // (cx, cy, cz) is the particle's own cell (inside the grid).  The offset may
 // lie outside [0, 1) (a stage point that left the cell); the cell it falls in
@@ -686,15 +713,7 @@ __device__ __forceinline__ float3 sample_local(const field_view& f, corner_cache
 {
   int ix = cx, iy = cy, iz = cz;
   float wx = ux, wy = uy, wz = uz;
-  if (!in_unit_cube(ux, uy, uz))
-  {
-    const float fx = floorf(ux), fy = floorf(uy), fz = floorf(uz);
-    ix += int(fx); iy += int(fy); iz += int(fz);
-    wx -= fx; wy -= fy; wz -= fz;
-    if (ix < 0) { ix = 0; wx = 0.0f; } else if (ix > f.nx - 2) { ix = f.nx - 2; wx = 1.0f; }
-    if (iy < 0) { iy = 0; wy = 0.0f; } else if (iy > f.ny - 2) { iy = f.ny - 2; wy = 1.0f; }
-    if (iz < 0) { iz = 0; wz = 0.0f; } else if (iz > f.nz - 2) { iz = f.nz - 2; wz = 1.0f; }
-  }
+  if (!in_unit_cube(ux, uy, uz)) find_cell(f, ix, iy, iz, wx, wy, wz);
   if (ix != k.ix || iy != k.iy || iz != k.iz) corner_load(f, k, ix, iy, iz);
   const float3 v = corner_eval(k, wx, wy, wz);
   const float2 vxy = __fmul2_rn(make_float2(f.inv_hx, f.inv_hy), make_float2(v.x, v.y));
@@ -704,12 +723,13 @@ __device__ __forceinline__ float3 sample_local(const field_view& f, corner_cache
 // Moves the offset back into [0, 1) and the cell accordingly.  For an offset
 // >= 1 the subtraction of its floor is exact; for a negative offset u, 1 + u
 // rounds to within 2^-25 and may give exactly 1 (the same point as offset 0
-// of the next cell).
+// of the next cell).  An axis inside [0, 1) is left as it is (its floor is 0): no
+// test, some lane of a warp leaves its cell at nearly every step.
 __device__ __forceinline__ void renormalize(local_position& p)
 {
-  if (!in_unit(p.ux)) { const float fl = floorf(p.ux); p.ix += int(fl); p.ux -= fl; }
-  if (!in_unit(p.uy)) { const float fl = floorf(p.uy); p.iy += int(fl); p.uy -= fl; }
-  if (!in_unit(p.uz)) { const float fl = floorf(p.uz); p.iz += int(fl); p.uz -= fl; }
+  take_floor(p.ix, p.ux);
+  take_floor(p.iy, p.uy);
+  take_floor(p.iz, p.uz);
 }
 
 __device__ __forceinline__ local_position to_local(const field_view& f, const float4& p)
@@ -834,15 +854,7 @@ __device__ __forceinline__ float3 sample_local_unsteady(const field_view& f, con
 {
   int ix = cx, iy = cy, iz = cz;
   float wx = ux, wy = uy, wz = uz;
-  if (!in_unit_cube(ux, uy, uz))
-  {
-    const float fx = floorf(ux), fy = floorf(uy), fz = floorf(uz);
-    ix += int(fx); iy += int(fy); iz += int(fz);
-    wx -= fx; wy -= fy; wz -= fz;
-    if (ix < 0) { ix = 0; wx = 0.0f; } else if (ix > f.nx - 2) { ix = f.nx - 2; wx = 1.0f; }
-    if (iy < 0) { iy = 0; wy = 0.0f; } else if (iy > f.ny - 2) { iy = f.ny - 2; wy = 1.0f; }
-    if (iz < 0) { iz = 0; wz = 0.0f; } else if (iz > f.nz - 2) { iz = f.nz - 2; wz = 1.0f; }
-  }
+  if (!in_unit_cube(ux, uy, uz)) find_cell(f, ix, iy, iz, wx, wy, wz);
   int slice;
   float wt;
   slice_of(ta, t, slice, wt);
@@ -895,7 +907,7 @@ __device__ __forceinline__ void local_unsteady_step(const field_view& f, const t
 // argument: its coefficients become immediates, its zeros vanish, and the
 // stages stay in registers (read from constant memory in runtime loops, the
 // stage array lived in local memory: 6.66 ms for the flow map of 96 x 90 x 101
-// vertices, 200 Dormand-Prince steps, now 3.3 ms).
+// vertices, 200 Dormand-Prince steps, now 3.2 ms).
 
 // acc += sum_{j = J}^{S - 1} a_Sj k_j
 template <int TABLEAU, int S, int J>
@@ -1003,9 +1015,9 @@ __device__ __forceinline__ void general_step_local(const field_view& f, corner_c
 // seeds: it looks every `steps` steps, and does so for `lanes` idle lanes at
 // least.  Both run for a few lanes while the rest of the warp waits, so they are
 // done for several lanes at once; waiting longer idles lanes.  256^3 flow map
-// (132 steps a seed) with 1 / 2 / 4 / 6 / 8 / 12 lanes: 56.4 / 53.8 / 52.6 / 52.6 /
-// 53.1 / 57.3 ms (57.9 ms with every lane refilled at once and 64-bit index
-// divisions).
+// (132 steps a seed, looking at every step) with 1 / 2 / 4 / 6 / 8 / 12 lanes: 56.4 /
+// 53.8 / 52.6 / 52.6 / 53.1 / 57.3 ms (57.9 ms with every lane refilled at once and
+// 64-bit index divisions); looking every eighth step: 51.0 ms.
 //
 // Launches of a few seeds per resident lane let a warp run its 32 seeds to the
 // end instead: refilled lanes are out of step, so that every warp, not only some,

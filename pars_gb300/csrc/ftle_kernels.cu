@@ -70,11 +70,12 @@ __device__ __forceinline__ void flow_step(const flow_map_args& a, corner_cache& 
 // One particle per lane, and lanes whose particles have ended take the next
 // seeds of their warp's pool (refill_rule): particles leave the grid
 // after very different step counts, and with one seed per thread a warp's lanes
-// idled until its longest particle ended.  Warps take pools of `pool`
-// consecutive seeds from a device counter.  Bound by instruction issue and the
+// idled until its longest particle ended.  Warps take pools of 32 consecutive
+// seeds from a device counter, as the batched engine does.  Bound by instruction issue and the
 // corner loads' L1 wavefronts, as the batched engine.  One seed per thread
-// against this: 5.51 -> 4.99 ms (frozen RK4, 150 x 128 x 141, 300 steps),
-// 657 -> 619 us (re-sampled RK4, 61 x 64 x 67, 120 steps, whole call).
+// against this: 5.51 -> 3.9 ms (frozen RK4, 150 x 128 x 141, 300 steps, with the
+// reciprocal divisions), 657 -> 549 us (re-sampled RK4, 61 x 64 x 67, 120 steps,
+// whole call).
 // Frozen steps need few registers once the corners are cached: seven CTAs of 128
 // per SM (72 registers) took 4.0 ms where 80 registers took 4.3 and 94 took 4.4
 // (150 x 128 x 141 vertices, 300 steps).  RK4 / Euler and Adams: five (96
@@ -85,7 +86,7 @@ constexpr int flow_min_ctas(int scheme)
 }
 
 template <int SCHEME>
-__global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(const __grid_constant__ flow_map_args a, int pool, refill_rule refill)
+__global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(const __grid_constant__ flow_map_args a, refill_rule refill)
 {
   constexpr unsigned full = 0xffffffffu;
   const long long total = (long long)a.px * a.py * a.pz;
@@ -138,10 +139,10 @@ __global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(co
           continue;
         }
         long long p = 0;
-        if (lane == 0) p = (long long)atomicAdd(a.next, (unsigned long long)pool);
+        if (lane == 0) p = (long long)atomicAdd(a.next, 32ULL);
         p = __shfl_sync(full, p, 0);
         if (p >= total) exhausted = true;
-        else { pool_next = p; pool_end = min(p + pool, total); }
+        else { pool_next = p; pool_end = min(p + 32, total); }
       }
       if (need == full) break;   // every lane idle, and the pools are exhausted
     }
@@ -191,15 +192,13 @@ cudaError_t flow_map_resident(flow_scheme scheme, int device, int* ctas)
   return e;
 }
 
-// `total` > 0 seeds on at most `resident` CTAs; pools as batch_pool_for cuts
-// them (256 seeds where every warp gets several pools, 32 where few do).
+// The lattice's seeds (at least one) on at most `resident` CTAs.
 cudaError_t launch_flow_map_kernel(const flow_map_args& a, flow_scheme scheme, int resident, cudaStream_t stream)
 {
   const long long total = (long long)a.px * a.py * a.pz;
-  int pool = (int)std::min<long long>(256, std::max<long long>(32, total / (4LL * resident * 4) / 32 * 32));
-  const unsigned grid = (unsigned)std::min<long long>(resident, (total + 4 * pool - 1) / (4 * pool));
+  const unsigned grid = (unsigned)std::min<long long>(resident, (total + 127) / 128);
   refill_rule refill = refill_for(total, resident * 128LL);
-  void* args[] = {(void*)&a, (void*)&pool, (void*)&refill};
+  void* args[] = {(void*)&a, (void*)&refill};
   return cudaLaunchKernel(flow_map_kernels[scheme], grid, 128, args, 0, stream);
 }
 
@@ -555,7 +554,7 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   f.ox = offset[0]; f.oy = offset[1]; f.oz = offset[2];
   f.hx = spacing[0]; f.hy = spacing[1]; f.hz = spacing[2];
   f.maxx = offset[0] + size[0]; f.maxy = offset[1] + size[1]; f.maxz = offset[2] + size[2];
-  set_reciprocals(f);
+  set_derived(f);
 
   // The counters (steps, seeds handed out) keep the previous call's values: clear them first.
   if (cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }

@@ -806,20 +806,10 @@ int class_of_job(const batch_job_device& j)
   return j.rule.frozen ? batch_frozen : (j.time.nt > 1 ? batch_unsteady : batch_steady);
 }
 
-long long pools_of(const batch_job_device& j) { return (j.seed_count + j.pool - 1) / j.pool; }
-
-// Cuts the jobs of one launch into pools of `pool` seeds, numbered through;
-// returns their number.
-long long number_pools(batch_job_device* jobs, int count, int pool)
+long long pools_of(const batch_job_device& j)
 {
-  long long pools = 0;
-  for (int k = 0; k < count; ++k)
-  {
-    jobs[k].pool = pool;
-    jobs[k].first_pool = pools;
-    pools += pools_of(jobs[k]);
-  }
-  return pools;
+  const int pool = batch_pool_seeds();
+  return (j.seed_count + pool - 1) / pool;
 }
 
 // Chooses the launch shape of job class c from `jobs` (all of class c, clocks
@@ -846,12 +836,14 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
   auto* device_jobs = ctx.batch_jobs.as<batch_job_device>();
   if (ctx.sm_count <= 0) PARS_CUDA(cudaDeviceGetAttribute(&ctx.sm_count, cudaDevAttrMultiProcessorCount, ctx.device));
   const long long probe = std::max(16384LL, 4LL * 2048LL * ctx.sm_count);
-  long long seeds = 0;
+  long long seeds = 0, pools = 0;
   for (int k = 0; k < count; ++k)
   {
     jobs[k].seed_count = std::min(jobs[k].seed_count, probe);
+    jobs[k].first_pool = pools;
     jobs[k].steps = counters + 1 + k;
     seeds += jobs[k].seed_count;
+    pools += pools_of(jobs[k]);
   }
   cudaEvent_t a, b;
   PARS_CUDA(cudaEventCreate(&a));
@@ -859,7 +851,6 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
   std::vector<float> fastest(batch_variant_count(), 0.0f);
   for (int v = 0; v < batch_variant_count(); ++v)
   {
-    const long long pools = number_pools(jobs.data(), count, batch_pool_for(ctx, c, v, seeds));
     for (int rep = 0; rep < 2; ++rep)
     {
       PARS_CUDA(cudaMemcpyAsync(device_jobs, jobs.data(), sizeof(batch_job_device) * count, cudaMemcpyHostToDevice, ctx.stream));
@@ -929,7 +920,7 @@ std::vector<unsigned long long> execute_batch(pars_gpu_context& ctx, std::vector
     if (variant < 0 && size[c] > 0 && ctx.batch_variant[c] < 0)
       tune_class(ctx, c, std::vector<batch_job_device>(queue.begin() + first[c], queue.begin() + first[c] + size[c]));
 
-  // The device queues: each job's seeds in pools of batch_pool_for(), numbered
+  // The device queues: each job's seeds in pools of batch_pool_seeds(), numbered
   // per class; counters 0 .. C-1 hand out the pools of the classes, counters
   // C.. count each job's steps.
   ctx.batch_jobs.reserve(sizeof(batch_job_device) * count);
@@ -938,16 +929,13 @@ std::vector<unsigned long long> execute_batch(pars_gpu_context& ctx, std::vector
   auto* device_jobs = ctx.batch_jobs.as<batch_job_device>();
   long long pools[C] = {}, seeds[C] = {};
   for (int c = 0; c < C; ++c)
-  {
-    if (size[c] == 0) continue;
     for (int k = first[c]; k < first[c] + size[c]; ++k)
     {
+      queue[k].first_pool = pools[c];
       queue[k].steps = counters + C + k;
+      pools[c] += pools_of(queue[k]);
       seeds[c] += queue[k].seed_count;
     }
-    const int shape = variant >= 0 ? variant : ctx.batch_variant[c];
-    pools[c] = number_pools(queue.data() + first[c], size[c], batch_pool_for(ctx, c, shape, seeds[c]));
-  }
   PARS_CUDA(cudaMemcpyAsync(device_jobs, queue.data(), sizeof(batch_job_device) * count, cudaMemcpyHostToDevice, ctx.stream));
   PARS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (count + C), ctx.stream));
   for (int c = 0; c < C; ++c)
@@ -1087,7 +1075,6 @@ long long engine_submit(pars_gpu_context& ctx, const batch_job_device& job)
   if (ctx.batch_variant[c] < 0) tune_class(ctx, c, {j});
   if (E.open == 0) E.variant = ctx.batch_variant[c];   // fixed while the class has work
   engine_reserve(ctx, E, int(E.jobs.size()) + 1);
-  j.pool = batch_pool_for(ctx, c, E.variant, j.seed_count);
   j.first_pool = E.total_pools;
   j.steps = E.counters.as<unsigned long long>() + 4 + E.jobs.size();
   E.total_pools += pools_of(j);

@@ -1,7 +1,6 @@
-"""Seed pools of the batched engine: a job's results are the same bits however
-its seeds are cut into pools (32 seeds where the launch is small, up to 256
-where every resident warp gets several pools), on the one-launch and the
-continuous engine, at the edges of a pool."""
+"""Seed pools of the batched engine: a job's results are the same bits whether it
+is alone in a launch (a warp's seeds run to the end), beside a large job (lanes
+refilled as particles end) or on the continuous engine, at the edges of a pool."""
 import numpy as np
 import pytest
 
@@ -37,7 +36,7 @@ def test_results_do_not_depend_on_the_pool_size(ctx, kind):
         p[:, 3] = 0.0
         return p
 
-    # a launch of 4 M seeds: pools of 256 seeds on any GPU with up to 152 SMs x 24 warps
+    # 4 M seeds: many rounds a lane on any GPU
     big = seeds(4 << 20)
     for n in (1, 31, 32, 33, 255, 257, 5000):
         s = seeds(n)
