@@ -160,14 +160,15 @@ __device__ __forceinline__ void add_steps(const trace_launch& a, unsigned int st
   if ((threadIdx.x & 31) == 0 && warp_steps) atomicAdd(a.steps, (unsigned long long)warp_steps);
 }
 
-// One particle per thread: for launches with no more particles than resident
-// lanes, where refilling cannot help and warp votes would only add latency.
+// One particle per thread, `lanes` of a warp's threads used: for launches with no
+// more particles than resident lanes, where refilling cannot help and warp votes
+// would only add latency.
 template <int MODE>
-__global__ void __launch_bounds__(128) trace_kernel(const __grid_constant__ trace_launch a)
+__global__ void __launch_bounds__(32) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
 {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = (long long)blockIdx.x * lanes + threadIdx.x;
   unsigned int steps = 0;
-  if (i < a.count)
+  if (int(threadIdx.x) < lanes && i < a.count)
   {
     lane_particle p;
     particle_start<MODE>(a, p, i);
@@ -616,6 +617,23 @@ unsigned int grid_for(long long work, int threads)
 }
 }
 
+namespace
+{
+// Particles per warp of a launch that does not fill the GPU: 32, or fewer (down
+// to 4) while the warps number at most 12 per SM.  A step waits for the slowest of
+// a warp's lanes, and whatever one lane needs (a new cell's corners) the whole
+// warp waits for, so few lanes a warp are faster as long as warps are few
+// (one launch of one particle per thread, 64^3 ABC: 512 particles of 1000 steps 456 us
+// with 32 lanes a warp, 394 with 4; 4096: 572, 500 with 4; 12167 of 800: 758, 721
+// with 8 or 16; 32768 fastest with 32 lanes: 634, 707 with 16.)
+int narrow_lanes(long long particles, int sms)
+{
+  int lanes = 4;
+  while (lanes < 32 && particles > 12LL * sms * lanes) lanes *= 2;
+  return lanes;
+}
+}
+
 void launch_trace(pars_gpu_context& ctx, const trace_launch& a)
 {
   if (a.count <= 0) return;
@@ -631,13 +649,12 @@ void launch_trace(pars_gpu_context& ctx, const trace_launch& a)
   launch_scope scope(ctx, "trace_streamlines");
   if (a.count <= resident_warps * 32)
   {
-    // every lane gets at most one particle: one per thread, narrow CTAs for
-    // small counts so that the work spreads over all SMs
-    const int threads = a.count <= 128LL * sms ? 32 : 128;
-    const unsigned grid = (unsigned)((a.count + threads - 1) / threads);
-    if (mode == trace_frozen)       trace_kernel<trace_frozen><<<grid, threads, 0, ctx.stream>>>(a);
-    else if (mode == trace_classic) trace_kernel<trace_classic><<<grid, threads, 0, ctx.stream>>>(a);
-    else                            trace_kernel<trace_general><<<grid, threads, 0, ctx.stream>>>(a);
+    // one particle per thread, one warp per CTA so that the work spreads over all SMs
+    const int lanes = narrow_lanes(a.count, sms);
+    const unsigned grid = (unsigned)((a.count + lanes - 1) / lanes);
+    if (mode == trace_frozen)       trace_kernel<trace_frozen><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    else if (mode == trace_classic) trace_kernel<trace_classic><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    else                            trace_kernel<trace_general><<<grid, 32, 0, ctx.stream>>>(a, lanes);
     return;
   }
   // pools of 256 particles when every resident warp gets several, else 32

@@ -1,0 +1,35 @@
+"""Launches that leave lanes of each warp unused: the same bits as the oracle on
+either side of every change of the lanes per warp."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import compare, gpu_curves
+
+pytestmark = pytest.mark.gpu
+
+
+def _edges():
+    import torch
+    fill = 12 * torch.cuda.get_device_properties(0).multi_processor_count
+    return [1, 3, 4 * fill, 4 * fill + 1, 8 * fill + 1, 16 * fill + 1]
+
+
+def _seeds(dtype, n, iterations):
+    p = np.zeros(n, dtype)
+    p["position"][:, :3] = np.random.default_rng(n).uniform(0.2, 6.1, (n, 3)).astype(np.float32)
+    p["remaining_iterations"] = iterations
+    p["vector_field_index"] = -1
+    return p
+
+
+@pytest.mark.parametrize("edge", range(6))
+def test_streamlines_match_the_oracle(ctx, port, edge):
+    from pars_gb300 import native, workloads as W
+    f = W.abc_field(17)
+    p = _seeds(native.PARTICLE_DTYPE, _edges()[edge], 22)
+    h = ctx.upload_field(f)
+    s = ctx.trace(h, p, 2, 0, 0.05)
+    expected = port.trace_single(f, p, 2, 0.05, "rgb", 0.5)
+    assert s["steps"] == expected.steps
+    compare(gpu_curves(ctx, s, "rgb"), expected.batches)
+    ctx.release_field(h)
