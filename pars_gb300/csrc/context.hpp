@@ -345,7 +345,6 @@ void launch_trace(pars_gpu_context& ctx, const trace_launch& a);
 // batches are rebuilt afterwards.
 constexpr int async_chunk = 32;
 constexpr int async_slab = 64;      // chunks a warp takes from the pool at once
-constexpr int async_claims = 32;    // segment ids a warp takes at once
 enum async_counter { async_head = 0, async_alloc = 1, async_done = 2, async_chunks = 3, async_steps = 4, async_counters = 5 };
 enum async_error { async_ok = 0, async_segments_full = 1, async_chunks_full = 2, async_wait_limit = 3 };
 struct async_launch
@@ -360,6 +359,8 @@ struct async_launch
   int*                seg_written;      // vertices written (slots of the reference's layout)
   int*                seg_kept;         // of them not invalid
   int*                seg_first_chunk;
+  long long           seeds;            // segments published before the launch
+  int                 lanes;            // lanes of a warp that trace (set by launch_async_trace)
   long long           capacity;         // segments
   float4*             chunks;           // async_chunk vertices each
   int*                chunk_next;
@@ -369,7 +370,7 @@ struct async_launch
 };
 // Launches the persistent kernel; returns its warps (each may leave part of a
 // chunk slab unused).
-long long launch_async_trace(pars_gpu_context& ctx, const async_launch& a, bool count_only = false);
+long long launch_async_trace(pars_gpu_context& ctx, async_launch& a, bool count_only = false);
 // Round-0 segments from ctx.particles_in / block_of (count particles).
 void launch_async_seed(pars_gpu_context& ctx, const async_launch& a, const pars_particle* particles, const int* block_of,
                        long long count);

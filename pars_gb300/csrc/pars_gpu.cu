@@ -596,6 +596,7 @@ bool run_rounds_async(pars_gpu_context& ctx, const std::vector<trace_block>& blo
   async_launch a {};
   a.blocks = device_blocks;
   a.rule = rule;
+  a.seeds = count;
   long long vertex_bound = 0;   // sum of remaining_iterations over the seeds, at most
   for (int b = 0; b < nblocks; ++b) vertex_bound += block_count[b] * std::max(1, block_max[b]);
   const long long warps = launch_async_trace(ctx, a, true);

@@ -224,14 +224,23 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(const __grid_cons
 
 // ---- Asynchronous rounds ---------------------------------------------------------
 // Every round of a partitioned domain in one persistent launch (no round
-// barrier): warps take segment ids in order, async_claims at a time, and hand
+// barrier): warps take segment ids in order, one per lane at a time, and hand
 // them to idle lanes; a lane starts its segment once the record is published,
 // and appends the continuation of a particle that leaves its block.  Vertex
 // chunks come from warp-private slabs of async_slab chunks, so the global
 // counters see one atomic per 32 claims or 64 chunks.  The launch ends when
 // every allocated segment is done (done read before allocated: a segment is
 // marked done only after its continuation was allocated and published).
-constexpr unsigned int async_wait_limit = 1u << 23;   // warp-wide idle polls (about 2 s with the sleeps)
+// What bounds the launch is its longest particle and every trip to L2 in its way:
+// lanes without a segment look for one every async_look turns only, and a warp with
+// nothing to trace polls less and less often (up to async_sleep ns apart), because
+// thousands of idle warps polling one counter slow every trip of the others.
+// 256^3 ABC in 64 blocks, re-sampled / frozen: 10 k seeds 4612 / 4403 us with a look
+// at every turn and polls 256 ns apart, 1525 / 1145 so; 100 k seeds 5963 / 5841,
+// 2285 / 1914; 512^3, 1 M seeds, the whole call: 22.8 ms, 19.1.
+constexpr int async_look = 16;
+constexpr unsigned int async_sleep = 8192;
+constexpr unsigned int async_wait_limit = 1u << 20;   // warp-wide idle polls (about 10 s with the pauses)
 
 // Device-scope memory-model accesses (PTX ld.acquire / ld.relaxed /
 // st.release): a segment's record is written before its ready flag is
@@ -284,12 +293,13 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
   const int lane = threadIdx.x & 31;
   const unsigned lanes_below = (1u << lane) - 1u;
   unsigned int steps = 0, waits = 0;
-  bool alive = false, finished = false;
+  bool alive = false, finished = lane >= a.lanes;
   long long claim = -1;
   unsigned long long known_allocated = 0;      // allocated segments, as last read
   long long pool_next = 0, pool_end = 0;       // warp-uniform: claimed ids not yet handed out
   long long slab_next = 0, slab_end = 0;       // warp-uniform: chunks not yet handed out
   int chunk = -1;
+  int turn = 0;
   lane_particle p;
   for (;;)
   {
@@ -302,7 +312,7 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
       if (k > left)
       {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(a.counters + async_head, (unsigned long long)async_claims);
+        if (lane == 0) base = atomicAdd(a.counters + async_head, (unsigned long long)a.lanes);
         fresh = (long long)__shfl_sync(full_mask, base, 0);
       }
       if (!alive && claim < 0 && !finished)
@@ -310,28 +320,24 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
         const long long mine = __popc(want & lanes_below);
         claim = mine < left ? pool_next + mine : fresh + (mine - left);
       }
-      if (k > left) { pool_next = fresh + (k - left); pool_end = fresh + async_claims; }
+      if (k > left) { pool_next = fresh + (k - left); pool_end = fresh + a.lanes; }
       else pool_next += k;
     }
-    // start a claimed segment once published; finish when every segment is
-    // done (done read before allocated: equal counts mean nothing is in flight)
-    if (claim >= 0)
+    // Start a claimed segment once published: the seeds are from the start, a
+    // continuation is looked for every async_look turns while other lanes of the
+    // warp trace (a look is two trips to L2, which those lanes would wait for at
+    // every step).  Finish when every segment is done (done read before
+    // allocated: equal counts mean nothing is in flight); that matters only to a
+    // warp with nothing to trace.
+    const bool idle = !__any_sync(full_mask, alive);
+    if (claim >= 0 && (claim < a.seeds || idle || turn % async_look == 0))
     {
-      if (claim >= a.capacity) { finished = true; claim = -1; }
-      else
+      bool published = claim < a.seeds;
+      if (!published && claim < a.capacity)
       {
         if ((unsigned long long)claim >= known_allocated) known_allocated = load_relaxed(a.counters + async_alloc);
-        if ((unsigned long long)claim < known_allocated)
-        {
-          if (load_acquire(a.seg_ready + claim))
-          {
-            async_start<MODE>(a, p, claim);
-            chunk = -1;
-            alive = true;
-            claim = -1;
-          }
-        }
-        else
+        if ((unsigned long long)claim < known_allocated) published = load_acquire(a.seg_ready + claim) != 0;
+        else if (idle)
         {
           const unsigned long long done = load_acquire(a.counters + async_done);
           const unsigned long long allocated = load_relaxed(a.counters + async_alloc);
@@ -339,14 +345,25 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
           if ((unsigned long long)claim >= allocated && done == allocated) { finished = true; claim = -1; }
         }
       }
+      if (claim >= a.capacity) { finished = true; claim = -1; }
+      if (published)
+      {
+        async_start<MODE>(a, p, claim);
+        chunk = -1;
+        alive = true;
+        claim = -1;
+      }
     }
+    ++turn;
     if (__all_sync(full_mask, finished)) break;
     if (!__any_sync(full_mask, alive))
     {
       // nothing to trace: stop on another lane's failure or after the wait limit
       if (load_acquire(a.error) != async_ok) break;
       if (++waits > async_wait_limit) { if (lane == 0) atomicCAS(a.error, async_ok, async_wait_limit); break; }
-      __nanosleep(256);
+      // (idle warps that poll without a pause load the counters' L2 slice, and
+      // every lane that looks for a continuation waits for it)
+      __nanosleep(min(async_sleep, 256u << min(waits - 1, 8u)));
       continue;
     }
     waits = 0;
@@ -665,7 +682,7 @@ void launch_trace(pars_gpu_context& ctx, const trace_launch& a)
   PARS_CUDA(cudaLaunchKernel(persistent, grid, 128, args, 0, ctx.stream));
 }
 
-long long launch_async_trace(pars_gpu_context& ctx, const async_launch& a, bool count_only)
+long long launch_async_trace(pars_gpu_context& ctx, async_launch& a, bool count_only)
 {
   const int mode = a.rule.frozen ? trace_frozen : (a.rule.scheme == scheme_classic ? trace_classic : trace_general);
   const void* kernel = mode == trace_frozen ? (const void*)async_trace_kernel<trace_frozen>
@@ -674,8 +691,14 @@ long long launch_async_trace(pars_gpu_context& ctx, const async_launch& a, bool 
   if (ctx.sm_count <= 0) PARS_CUDA(cudaDeviceGetAttribute(&ctx.sm_count, cudaDevAttrMultiProcessorCount, ctx.device));
   int& per_sm = ctx.async_ctas_per_sm[mode];
   if (per_sm < 0) PARS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 128, 0));
-  // as many CTAs as are resident at once: lanes wait for segments that others publish
-  const unsigned grid = (unsigned)(std::max(per_sm, 1) * ctx.sm_count);
+  // At most as many CTAs as are resident at once: lanes wait for segments that
+  // others publish.  A particle has one segment at a time, so as many lanes as
+  // seeds always suffice; few seeds leave lanes of every warp unused, which
+  // spreads them over more warps (narrow_lanes).
+  const long long resident = (long long)std::max(per_sm, 1) * ctx.sm_count;
+  a.lanes = narrow_lanes(a.seeds, ctx.sm_count);
+  const long long needed = ((a.seeds + a.lanes - 1) / a.lanes + 3) / 4;
+  const unsigned grid = (unsigned)std::max<long long>(1, std::min(resident, needed));
   if (count_only) return (long long)grid * 4;
   launch_scope scope(ctx, "trace_async");
   void* args[] = {(void*)&a};

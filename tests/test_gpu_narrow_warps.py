@@ -33,3 +33,23 @@ def test_streamlines_match_the_oracle(ctx, port, edge):
     assert s["steps"] == expected.steps
     compare(gpu_curves(ctx, s, "rgb"), expected.batches)
     ctx.release_field(h)
+
+
+@pytest.mark.parametrize("edge", range(6))
+def test_domain_matches_the_oracle(ctx, port, edge):
+    from pars_gb300 import native, workloads as W
+    f = W.abc_field(17)
+    ranks = 8
+    info = port.partition(ranks, 0, f.dims)
+    p = _seeds(native.PARTICLE_DTYPE, _edges()[edge], 22)
+    extent = (f.spacing * info["block"]).astype(np.float32)
+    multi = np.minimum((p["position"][:, :3] / extent).astype(np.int64), info["grid"] - 1)
+    owner = (multi[:, 0] * info["grid"][1] + multi[:, 1]) * info["grid"][2] + multi[:, 2]
+    p = p[np.argsort(owner, kind="stable")]
+    offsets = np.concatenate([[0], np.cumsum(np.bincount(owner, minlength=ranks))]).astype(np.int64)
+    d = ctx.domain_create(f, ranks)
+    s = ctx.trace_domain(d, p, offsets, 2, 0, 0.05)
+    expected = port.trace_multi(f, ranks, offsets, p, 2, 0.05, "rgb", 0.5)
+    assert s["steps"] == expected.steps
+    compare(gpu_curves(ctx, s, "rgb"), expected.batches)
+    ctx.domain_release(d)
