@@ -82,6 +82,8 @@ private:
 struct field_entry
 {
   device_buffer data;          // float4 [slices][X][Y][Z]
+  int           z_pairs = 0;   // field_view::z_pairs
+  device_buffer paired;        // a flow map's copy with z_pairs, once it has been traced through
   int           shape[3];
   float         offset[3], size[3], spacing[3];
   int           slices = 1;    // time slices (1 = steady)
@@ -104,6 +106,7 @@ struct field_entry
     v.hx = spacing[0]; v.hy = spacing[1]; v.hz = spacing[2];
     v.maxx = offset[0] + size[0]; v.maxy = offset[1] + size[1]; v.maxz = offset[2] + size[2];
     set_derived(v);
+    v.z_pairs = z_pairs;
     return v;
   }
 };
@@ -299,7 +302,10 @@ void take_profile(pars_gpu_context& ctx, std::map<std::string, profile_entry>& i
 step_rule make_step_rule(int integrator, int stage_mode, float h);
 
 // Kernel launchers (defined in the *_kernels.cu translation units).
-void launch_pack_field(pars_gpu_context& ctx, const float* xyz, float4* out, long long count);
+// count vertices as float4 with z_pairs; plane: vertices between x and x + 1
+void launch_pack_field(pars_gpu_context& ctx, const float* xyz, float4* out, long long count, long long plane);
+// the same from float4 vertices (w not read)
+void launch_pair_field(pars_gpu_context& ctx, const float4* data, float4* out, long long count, long long plane);
 void launch_unpack_field(pars_gpu_context& ctx, const float4* data, float* xyz, long long count);
 void launch_field_sample(pars_gpu_context& ctx, const field_view& f, const float4* positions, long long n, uint8_t* inside, float* velocity);
 void launch_seed_generate(pars_gpu_context& ctx, const float offset[3], const float stride[3], const int per_dimension[3],

@@ -21,8 +21,12 @@
 
 namespace pars
 {
-// A block of a vector field, resident as float4 (x, y, z, 0) per vertex,
-// [X][Y][Z] in C order (z fastest), like pa::vector_field::data.
+// A block of a vector field, resident as float4 per vertex, [X][Y][Z] in C order
+// (z fastest), like pa::vector_field::data: (x, y, z, the z component of the
+// vertex at x + 1) when z_pairs, which every uploaded field and domain block has.
+// A flow map keeps its residual codes in the last lane instead: the FTLE reads it as
+// it is, and what is traced through it is its copy with z_pairs (velocity_view; a
+// test of the flag at the corner loads cost 2 to 4 % of a flow map).
 struct field_view
 {
   const float4* data;
@@ -32,6 +36,7 @@ struct field_view
   float         maxx, maxy, maxz;  // offset + size (block-exit face tests)
   float         inv_hx, inv_hy, inv_hz;  // RN(1 / spacing)
   int           fast_division;           // 1: quotient_rn holds for this spacing (divides_fast)
+  int           z_pairs;                 // 1: w holds the z component of the vertex at x + 1
 };
 
 // Whether x / h may be formed with quotient_rn for this spacing: with h in
@@ -216,40 +221,36 @@ __device__ __forceinline__ float lerp_fast(float a, float b, float w) { return f
 // ---- Register-cached cell (re-sampled path) ----------------------------------
 // A particle moves up to about a cell per RK4 step, so most stage samples fall
 // into the cell sampled last.  The lane keeps that cell's eight corners in
-// registers, and only a change of cell issues the eight 16-byte corner loads.
+// registers, and only a change of cell issues the eight corner loads.
 // Within a warp some lane changes cell at almost every sample, so whatever
 // runs only for the lanes that change cell costs the whole warp nearly every
 // sample: that part is kept to the loads, and the interpolation (lerps along
 // z, then y, then x) runs once for all lanes together.
+// The z components of c0yz and c1yz lie side by side in c0yz's register pair
+// (z, w), as the field stores them, so they go through the packed lerps as they
+// were loaded, and the corners at x + 1 are 8-byte loads.  256^3 FTLE flow map:
+// 4 % less than eight 16-byte loads and scalar lerps of z (49.9 -> 48.0 ms with the
+// FTLE), frozen flow maps 7 %, pathlines 3 %.
 struct corner_cache
 {
   int    ix = -1, iy = -1, iz = -1;
-  float3 c000, c001, c010, c011, c100, c101, c110, c111;
+  float4 c000, c001, c010, c011;   // w: the z component of the corner at x + 1
+  float2 c100, c101, c110, c111;
 };
-
-__device__ __forceinline__ float3 xyz_of(const float4& v) { return make_float3(v.x, v.y, v.z); }
 
 __device__ __forceinline__ void corner_load(const field_view& f, corner_cache& k, int ix, int iy, int iz)
 {
   const long long syz = (long long)f.ny * f.nz;
   const float4* base = f.data + ((long long)ix * f.ny + iy) * f.nz + iz;
   k.ix = ix; k.iy = iy; k.iz = iz;
-  k.c000 = xyz_of(__ldg(base));
-  k.c001 = xyz_of(__ldg(base + 1));
-  k.c010 = xyz_of(__ldg(base + f.nz));
-  k.c011 = xyz_of(__ldg(base + f.nz + 1));
-  k.c100 = xyz_of(__ldg(base + syz));
-  k.c101 = xyz_of(__ldg(base + syz + 1));
-  k.c110 = xyz_of(__ldg(base + syz + f.nz));
-  k.c111 = xyz_of(__ldg(base + syz + f.nz + 1));
-}
-
-__device__ __forceinline__ float corner_eval1(float c000, float c001, float c010, float c011, float c100, float c101,
-                                              float c110, float c111, float wx, float wy, float wz)
-{
-  const float c00 = lerp_fast(c000, c001, wz), c01 = lerp_fast(c010, c011, wz);
-  const float c10 = lerp_fast(c100, c101, wz), c11 = lerp_fast(c110, c111, wz);
-  return lerp_fast(lerp_fast(c00, c01, wy), lerp_fast(c10, c11, wy), wx);
+  k.c000 = __ldg(base);
+  k.c001 = __ldg(base + 1);
+  k.c010 = __ldg(base + f.nz);
+  k.c011 = __ldg(base + f.nz + 1);
+  k.c100 = __ldg(reinterpret_cast<const float2*>(base + syz));
+  k.c101 = __ldg(reinterpret_cast<const float2*>(base + syz + 1));
+  k.c110 = __ldg(reinterpret_cast<const float2*>(base + syz + f.nz));
+  k.c111 = __ldg(reinterpret_cast<const float2*>(base + syz + f.nz + 1));
 }
 
 // The reference's blend (lerp_exact along z, then y, then x) of a cached cell:
@@ -258,8 +259,8 @@ __device__ __forceinline__ float3 blend8_cached(const corner_cache& k, float wx,
 {
   const float4 c000 = make_float4(k.c000.x, k.c000.y, k.c000.z, 0.f), c001 = make_float4(k.c001.x, k.c001.y, k.c001.z, 0.f);
   const float4 c010 = make_float4(k.c010.x, k.c010.y, k.c010.z, 0.f), c011 = make_float4(k.c011.x, k.c011.y, k.c011.z, 0.f);
-  const float4 c100 = make_float4(k.c100.x, k.c100.y, k.c100.z, 0.f), c101 = make_float4(k.c101.x, k.c101.y, k.c101.z, 0.f);
-  const float4 c110 = make_float4(k.c110.x, k.c110.y, k.c110.z, 0.f), c111 = make_float4(k.c111.x, k.c111.y, k.c111.z, 0.f);
+  const float4 c100 = make_float4(k.c100.x, k.c100.y, k.c000.w, 0.f), c101 = make_float4(k.c101.x, k.c101.y, k.c001.w, 0.f);
+  const float4 c110 = make_float4(k.c110.x, k.c110.y, k.c010.w, 0.f), c111 = make_float4(k.c111.x, k.c111.y, k.c011.w, 0.f);
   return blend8(c000, c001, c010, c011, c100, c101, c110, c111, wx, wy, wz);
 }
 
@@ -286,9 +287,8 @@ __device__ __forceinline__ float2 lerp_fast2(float2 a, float2 b, float2 w)
 }
 
 // The trilinear blend of a cached cell with lerp_fast along z, then y, then x:
-// x and y components through the packed pair (7 paired lerps instead of 14
-// scalar ones), z through the scalar blend.  Measured on the 256^3 FTLE
-// workload: 4.4 % less kernel time than three scalar blends, same end points.
+// x and y as a packed pair (7 paired lerps), the z components of the corners at x
+// and x + 1 as another (3 paired lerps and the scalar one along x).
 __device__ __forceinline__ float3 corner_eval(const corner_cache& k, float wx, float wy, float wz)
 {
   const float2 Wz = make_float2(wz, wz), Wy = make_float2(wy, wy), Wx = make_float2(wx, wx);
@@ -297,8 +297,10 @@ __device__ __forceinline__ float3 corner_eval(const corner_cache& k, float wx, f
   const float2 c10 = lerp_fast2(make_float2(k.c100.x, k.c100.y), make_float2(k.c101.x, k.c101.y), Wz);
   const float2 c11 = lerp_fast2(make_float2(k.c110.x, k.c110.y), make_float2(k.c111.x, k.c111.y), Wz);
   const float2 xy = lerp_fast2(lerp_fast2(c00, c01, Wy), lerp_fast2(c10, c11, Wy), Wx);
-  return make_float3(xy.x, xy.y,
-                     corner_eval1(k.c000.z, k.c001.z, k.c010.z, k.c011.z, k.c100.z, k.c101.z, k.c110.z, k.c111.z, wx, wy, wz));
+  const float2 z0 = lerp_fast2(make_float2(k.c000.z, k.c000.w), make_float2(k.c001.z, k.c001.w), Wz);
+  const float2 z1 = lerp_fast2(make_float2(k.c010.z, k.c010.w), make_float2(k.c011.z, k.c011.w), Wz);
+  const float2 z = lerp_fast2(z0, z1, Wy);
+  return make_float3(xy.x, xy.y, lerp_fast(z.x, z.y, wx));
 }
 
 // Eigen isZero() with its default precision (NumTraits<float>::dummy_precision).

@@ -1,4 +1,4 @@
-// Field packing (xyz FP32 -> float4, the repack of data_io.cpp:99-106), field
+// Field packing (xyz FP32 -> float4 with z_pairs, for the repack of data_io.cpp:99-106), field
 // sampling (vector_field::contains + ::interpolate at given positions) and
 // lattice seeding (seed_generator::generate, seed_generator.cpp:9-21).
 #include "context.hpp"
@@ -7,11 +7,21 @@ namespace pars
 {
 namespace
 {
-__global__ void pack_field_kernel(const float* __restrict__ xyz, float4* __restrict__ out, long long count)
+__global__ void pack_field_kernel(const float* __restrict__ xyz, float4* __restrict__ out, long long count, long long plane)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  out[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], 0.0f);
+  // (the last x plane's w is never read)
+  out[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], i + plane < count ? xyz[3 * (i + plane) + 2] : 0.0f);
+}
+
+__global__ void pair_field_kernel(const float4* __restrict__ data, float4* __restrict__ out, long long count, long long plane)
+{
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= count) return;
+  float4 v = data[i];
+  v.w = i + plane < count ? data[i + plane].z : 0.0f;
+  out[i] = v;
 }
 
 __global__ void unpack_field_kernel(const float4* __restrict__ data, float* __restrict__ xyz, long long count)
@@ -66,11 +76,18 @@ __global__ void seed_kernel(const seed_args a)
 }
 }
 
-void launch_pack_field(pars_gpu_context& ctx, const float* xyz, float4* out, long long count)
+void launch_pack_field(pars_gpu_context& ctx, const float* xyz, float4* out, long long count, long long plane)
 {
   if (count <= 0) return;
   launch_scope scope(ctx, "field_pack");
-  pack_field_kernel<<<(unsigned)((count + 255) / 256), 256, 0, ctx.stream>>>(xyz, out, count);
+  pack_field_kernel<<<(unsigned)((count + 255) / 256), 256, 0, ctx.stream>>>(xyz, out, count, plane);
+}
+
+void launch_pair_field(pars_gpu_context& ctx, const float4* data, float4* out, long long count, long long plane)
+{
+  if (count <= 0) return;
+  launch_scope scope(ctx, "field_pair");
+  pair_field_kernel<<<(unsigned)((count + 255) / 256), 256, 0, ctx.stream>>>(data, out, count, plane);
 }
 
 void launch_unpack_field(pars_gpu_context& ctx, const float4* data, float* xyz, long long count)

@@ -288,6 +288,7 @@ __device__ __forceinline__ float largest_eigenvalue(float c00, float c11, float 
 struct ftle_args
 {
   const float4* flow;
+  unsigned int  codes;            // ~0: the w lanes hold residual codes, 0: they do not
   int           nx, ny, nz;
   float         width[3], inverse_width[3];   // 2 h per axis and its reciprocal
   float         inverse_time;     // 1 / |T|
@@ -333,12 +334,12 @@ __global__ void __launch_bounds__(256) ftle_kernel(const ftle_args a)
     if (ext[j] == 1) { J[0][j] = J[1][j] = J[2][j] = 0.0f; continue; }
     const bool first = idx[j] == 0, last = idx[j] == ext[j] - 1;
     const long long lo = first ? i : i - stride[j], hi = last ? i : i + stride[j];
-    // positions with their sub-ulp residuals (w = 0: none); the FP32
+    // positions with their sub-ulp residuals (code 0: none); the FP32
     // difference of neighbouring coordinates is exact where they lie within a
     // factor of two of each other (Sterbenz), the residuals' difference is
     // added to it
     const float4 A = __ldg(a.flow + lo), B = __ldg(a.flow + hi);
-    const unsigned wa = __float_as_uint(A.w), wb = __float_as_uint(B.w);
+    const unsigned wa = __float_as_uint(A.w) & a.codes, wb = __float_as_uint(B.w) & a.codes;
     // a one-sided difference is doubled (exactly), so every axis divides by 2 h
     const float twice = first || last ? 2.0f : 1.0f;
     J[0][j] = quotient(twice * coordinate_difference(B.x, wb, A.x, wa, 0), a.width[j], a.inverse_width[j]);
@@ -417,7 +418,7 @@ const unsigned long long* launch_flow_map(pars_gpu_context& ctx, const field_vie
 void launch_ftle(pars_gpu_context& ctx, const field_view& flow, double time, int mode, float* out)
 {
   ftle_args a;
-  a.flow = flow.data; a.nx = flow.nx; a.ny = flow.ny; a.nz = flow.nz;
+  a.flow = flow.data; a.codes = flow.z_pairs ? 0u : ~0u; a.nx = flow.nx; a.ny = flow.ny; a.nz = flow.nz;
   set_widths(a, flow.hx, flow.hy, flow.hz);
   a.inverse_time = float(1.0 / fabs(time));
   a.mode = mode;
@@ -445,10 +446,11 @@ constexpr long long no_alloc_max_voxels = 1LL << 18;   // 64^3
 constexpr long long no_alloc_entries = 2 * no_alloc_max_voxels + 16;   // field | flow map | counter
 static __device__ __align__(256) float4 no_alloc_scratch[no_alloc_entries];
 
-__global__ void pack_into_scratch_kernel(const float* __restrict__ xyz, float4* __restrict__ out, long long count)
+__global__ void pack_into_scratch_kernel(const float* __restrict__ xyz, float4* __restrict__ out, long long count, long long plane)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) out[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], 0.0f);
+  if (i < count)   // field_view::z_pairs
+    out[i] = make_float4(xyz[3 * i], xyz[3 * i + 1], xyz[3 * i + 2], i + plane < count ? xyz[3 * (i + plane) + 2] : 0.0f);
 }
 
 __global__ void steps_to_int64_kernel(const unsigned long long* __restrict__ counter, int64_t* __restrict__ out)
@@ -555,10 +557,11 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   f.hx = spacing[0]; f.hy = spacing[1]; f.hz = spacing[2];
   f.maxx = offset[0] + size[0]; f.maxy = offset[1] + size[1]; f.maxz = offset[2] + size[2];
   set_derived(f);
+  f.z_pairs = 1;
 
   // The counters (steps, seeds handed out) keep the previous call's values: clear them first.
   if (cudaMemsetAsync(counter, 0, 2 * sizeof(unsigned long long), s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
-  pack_into_scratch_kernel<<<(unsigned)((voxels + 255) / 256), 256, 0, s>>>(device_xyz, field_data, voxels);
+  pack_into_scratch_kernel<<<(unsigned)((voxels + 255) / 256), 256, 0, s>>>(device_xyz, field_data, voxels, (long long)shape[1] * shape[2]);
   if (cudaGetLastError() != cudaSuccess) return PARS_ERR_CUDA;
 
   flow_map_args a;
@@ -571,7 +574,7 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   if (launch_flow_map_kernel(a, scheme, resident, s) != cudaSuccess) { (void)cudaGetLastError(); return PARS_ERR_CUDA; }
 
   ftle_args t;
-  t.flow = flow; t.nx = shape[0]; t.ny = shape[1]; t.nz = shape[2];
+  t.flow = flow; t.codes = ~0u; t.nx = shape[0]; t.ny = shape[1]; t.nz = shape[2];
   set_widths(t, spacing[0], spacing[1], spacing[2]);
   t.inverse_time = float(1.0 / fabs(double(time)));
   t.mode = mode;

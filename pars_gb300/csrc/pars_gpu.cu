@@ -37,7 +37,7 @@ void for_each_scratch(context_type& c, visit_type&& visit)
 long long pars_gpu_context::held_bytes() const
 {
   long long total = 0;
-  for (auto& f : fields) total += (long long)f.second->data.bytes();
+  for (auto& f : fields) total += (long long)(f.second->data.bytes() + f.second->paired.bytes());
   for (auto& d : domains) total += (long long)d.second->device_blocks.bytes();
   for_each_scratch(*this, [&](const pars::device_buffer& b) { total += (long long)b.bytes(); });
   return total + (long long)buffer_cache_bytes;
@@ -214,6 +214,23 @@ void check_field_args(const int32_t shape[3], const float spacing[3])
   PARS_REQUIRE((long long)shape[0] * shape[1] * shape[2] < (1LL << 40), "field too large");
 }
 
+// The field as tracing reads it (with z_pairs); a flow map gets its copy at the
+// first call, on the context's stream.
+field_view velocity_view(pars_gpu_context& ctx, field_entry& f)
+{
+  field_view v = f.view();
+  if (f.z_pairs) return v;
+  if (f.paired.bytes() == 0)
+  {
+    const long long plane = (long long)f.shape[1] * f.shape[2], count = plane * f.shape[0];
+    f.paired = acquire_buffer(ctx, sizeof(float4) * count);
+    launch_pair_field(ctx, f.data.as<const float4>(), f.paired.as<float4>(), count, plane);
+  }
+  v.data = f.paired.as<const float4>();
+  v.z_pairs = 1;
+  return v;
+}
+
 int32_t add_field(pars_gpu_context& ctx, std::unique_ptr<field_entry> entry)
 {
   const int32_t handle = ctx.next_handle++;
@@ -221,6 +238,7 @@ int32_t add_field(pars_gpu_context& ctx, std::unique_ptr<field_entry> entry)
   return handle;
 }
 
+// The entry of a field that is packed from xyz triples.
 std::unique_ptr<field_entry> make_field(const int32_t shape[3], const float offset[3], const float size[3], const float spacing[3])
 {
   auto entry = std::make_unique<field_entry>();
@@ -231,6 +249,7 @@ std::unique_ptr<field_entry> make_field(const int32_t shape[3], const float offs
     entry->spacing[i] = spacing[i];
     entry->size[i] = size ? size[i] : float(shape[i]) * spacing[i];
   }
+  entry->z_pairs = 1;   // launch_pack_field
   return entry;
 }
 
@@ -771,10 +790,10 @@ bool run_rounds_async(pars_gpu_context& ctx, const std::vector<trace_block>& blo
 }
 
 // Single block: one trace_block with no neighbours, kept in a small device array.
-const trace_block* single_block(pars_gpu_context& ctx, const field_entry& f, std::vector<trace_block>& blocks)
+const trace_block* single_block(pars_gpu_context& ctx, field_entry& f, std::vector<trace_block>& blocks)
 {
   trace_block b;
-  b.field = f.view();
+  b.field = velocity_view(ctx, f);
   for (int i = 0; i < 6; ++i) b.neighbor[i] = -1;
   blocks.assign(1, b);
   ctx.single_block.reserve(sizeof(trace_block));
@@ -1230,7 +1249,7 @@ batch_job_device device_job(pars_gpu_context& ctx, const pars_gpu_batch_job& in)
 {
   auto& f = find_field(ctx, in.field);
   batch_job_device d {};
-  d.field = f.view();
+  d.field = velocity_view(ctx, f);
   d.time = f.time();
   d.rule = make_rule(in.integrator, in.stage_mode, in.step_size);
   if (d.rule.frozen && d.time.nt > 1)
@@ -1341,7 +1360,7 @@ int32_t pars_gpu_field_upload(pars_gpu_context* ctx, const float* xyz, const int
     ctx->staging.reserve(sizeof(float) * 3 * count);
     entry->data = acquire_buffer(*ctx, sizeof(float4) * count);
     PARS_CUDA(cudaMemcpyAsync(ctx->staging.get(), xyz, sizeof(float) * 3 * count, cudaMemcpyHostToDevice, ctx->stream));
-    launch_pack_field(*ctx, ctx->staging.as<const float>(), entry->data.as<float4>(), count);
+    launch_pack_field(*ctx, ctx->staging.as<const float>(), entry->data.as<float4>(), count, (long long)shape[1] * shape[2]);
     // the caller may reuse or free its buffer once the call returns
     PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     *field = add_field(*ctx, std::move(entry));
@@ -1357,7 +1376,7 @@ int32_t pars_gpu_field_upload_device(pars_gpu_context* ctx, const float* device_
     auto entry = make_field(shape, offset, size, spacing);
     const long long count = (long long)shape[0] * shape[1] * shape[2];
     entry->data = acquire_buffer(*ctx, sizeof(float4) * count);
-    launch_pack_field(*ctx, device_xyz, entry->data.as<float4>(), count);
+    launch_pack_field(*ctx, device_xyz, entry->data.as<float4>(), count, (long long)shape[1] * shape[2]);
     // the caller may reuse or free its buffer once the call returns
     PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     *field = add_field(*ctx, std::move(entry));
@@ -1378,7 +1397,7 @@ int32_t pars_gpu_unsteady_field_upload(pars_gpu_context* ctx, const float* xyz, 
     ctx->staging.reserve(sizeof(float) * 3 * count);
     entry->data = acquire_buffer(*ctx, sizeof(float4) * count);
     PARS_CUDA(cudaMemcpyAsync(ctx->staging.get(), xyz, sizeof(float) * 3 * count, cudaMemcpyHostToDevice, ctx->stream));
-    launch_pack_field(*ctx, ctx->staging.as<const float>(), entry->data.as<float4>(), count);
+    launch_pack_field(*ctx, ctx->staging.as<const float>(), entry->data.as<float4>(), count, (long long)shape[1] * shape[2]);
     // the caller may reuse or free its buffer once the call returns
     PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     *field = add_field(*ctx, std::move(entry));
@@ -1397,7 +1416,7 @@ int32_t pars_gpu_unsteady_field_upload_device(pars_gpu_context* ctx, const float
     entry->slices = slices; entry->t0 = t0; entry->slice_dt = slice_dt;
     const long long count = (long long)shape[0] * shape[1] * shape[2] * slices;
     entry->data = acquire_buffer(*ctx, sizeof(float4) * count);
-    launch_pack_field(*ctx, device_xyz, entry->data.as<float4>(), count);
+    launch_pack_field(*ctx, device_xyz, entry->data.as<float4>(), count, (long long)shape[1] * shape[2]);
     // the caller may reuse or free its buffer once the call returns
     PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     *field = add_field(*ctx, std::move(entry));
@@ -1415,6 +1434,7 @@ int32_t pars_gpu_field_release(pars_gpu_context* ctx, int32_t field)
     // Work queued on the context's stream may still read the buffer; anything
     // that reuses it is queued behind that work on the same stream.
     recycle_buffer(*ctx, std::move(it->second->data));
+    recycle_buffer(*ctx, std::move(it->second->paired));
     ctx->fields.erase(it);
   });
 }
@@ -1548,6 +1568,7 @@ int32_t build_domain(pars_gpu_context* ctx, const float* device_xyz, const int32
     for (int i = 0; i < 3; ++i) PARS_REQUIRE(f->shape[i] >= 2, "blocks must be at least 2 voxels wide");
     f->data = acquire_buffer(*ctx, sizeof(float4) * (std::size_t)f->shape[0] * f->shape[1] * f->shape[2]);
     launch_extract_block(*ctx, device_xyz, domain_size, info.offset, f->shape, f->data.as<float4>());
+    f->z_pairs = 1;
     trace_block b;
     b.field = f->view();
     for (int face = 0; face < 6; ++face) b.neighbor[face] = info.neighbor_rank[face];
@@ -1667,7 +1688,7 @@ int32_t pars_gpu_domain_assemble(pars_gpu_context* ctx, int32_t ranks, const int
         PARS_REQUIRE(f.shape[i] == info.ghosted_block_size[i],
                      "field of rank " + std::to_string(r) + " is not its ghosted block of the partition");
       trace_block b;
-      b.field = f.view();
+      b.field = velocity_view(*ctx, f);
       for (int face = 0; face < 6; ++face) b.neighbor[face] = info.neighbor_rank[face];
       entry->blocks.push_back(b);
       entry->fields.push_back(fields[r]);
@@ -1916,7 +1937,7 @@ int32_t pars_gpu_flow_map_generate(pars_gpu_context* ctx, int32_t field, int32_t
       // steps/s on the 256^3 flow map), the iterations <= 1 case, where every
       // voxel keeps its seed position, and the re-sampled stages of the
       // general schemes.
-      const unsigned long long* counter = launch_flow_map(*ctx, f.view(), rule, iterations, f.offset, entry->spacing, seeds, entry->shape,
+      const unsigned long long* counter = launch_flow_map(*ctx, velocity_view(*ctx, f), rule, iterations, f.offset, entry->spacing, seeds, entry->shape,
                                                           entry->data.as<float4>());
       if (steps)
       {
@@ -1931,7 +1952,7 @@ int32_t pars_gpu_flow_map_generate(pars_gpu_context* ctx, int32_t field, int32_t
       // Re-sampled RK4 / Euler: one job of the persistent batched engine.
       std::vector<batch_job_device> job(1);
       batch_job_device& d = job[0];
-      d.field = f.view();
+      d.field = velocity_view(*ctx, f);
       d.time = f.time();
       d.rule = rule;
       d.max_steps = iterations - 1;

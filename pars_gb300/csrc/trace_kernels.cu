@@ -625,7 +625,8 @@ __global__ void extract_block_kernel(const float* __restrict__ domain, int dy, i
   const int y = int((i / sz) % sy);
   const int x = int(i / ((long long)sz * sy));
   const long long g = ((long long)(ox + x) * dy + (oy + y)) * dz + (oz + z);
-  out[i] = make_float4(domain[3 * g], domain[3 * g + 1], domain[3 * g + 2], 0.0f);
+  out[i] = make_float4(domain[3 * g], domain[3 * g + 1], domain[3 * g + 2],
+                       x + 1 < sx ? domain[3 * (g + (long long)dy * dz) + 2] : 0.0f);   // field_view::z_pairs
 }
 
 unsigned int grid_for(long long work, int threads)
