@@ -637,15 +637,17 @@ unsigned int grid_for(long long work, int threads)
 
 namespace
 {
-// Particles per warp of a launch that does not fill the GPU: 32, or fewer (down
-// to 4) while the warps number at most 12 per SM.  A step waits for the slowest of
-// a warp's lanes, and whatever one lane needs (a new cell's corners) the whole
-// warp waits for, so few lanes a warp are faster as long as warps are few
-// (one launch of one particle per thread, 64^3 ABC: 512 particles of 1000 steps 456 us
-// with 32 lanes a warp, 394 with 4; 4096: 572, 500 with 4; 12167 of 800: 758, 721
-// with 8 or 16; 32768 fastest with 32 lanes: 634, 707 with 16.)
+// Particles per warp of a launch that does not fill the GPU: one while that gives
+// at most a warp per scheduler, else 4, 8, 16 or 32, as few as keep the warps
+// below 12 per SM.  A step waits for the slowest of a warp's lanes, and whatever
+// one lane needs (a new cell's corners) the whole warp waits for, so few lanes a
+// warp are faster as long as warps are few (64^3 ABC, 512 particles of 1000 steps:
+// 456 us with 32 lanes a warp, 380 with 4, 331 with one; 4096: 572, 481 with 4;
+// 12167 of 800: 758, 695 with 8; 32768 fastest with 32: 605, 669 with 16; gyre of
+// 198^3, 1331 particles: 1050 with 4, 1165 with one).
 int narrow_lanes(long long particles, int sms)
 {
+  if (particles <= 4LL * sms) return 1;
   int lanes = 4;
   while (lanes < 32 && particles > 12LL * sms * lanes) lanes *= 2;
   return lanes;

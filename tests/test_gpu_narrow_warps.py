@@ -10,8 +10,9 @@ pytestmark = pytest.mark.gpu
 
 def _edges():
     import torch
-    fill = 12 * torch.cuda.get_device_properties(0).multi_processor_count
-    return [1, 3, 4 * fill, 4 * fill + 1, 8 * fill + 1, 16 * fill + 1]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    fill = 12 * sms
+    return [1, 4 * sms, 4 * sms + 1, 4 * fill, 4 * fill + 1, 8 * fill + 1, 16 * fill + 1]
 
 
 def _seeds(dtype, n, iterations):
@@ -22,7 +23,7 @@ def _seeds(dtype, n, iterations):
     return p
 
 
-@pytest.mark.parametrize("edge", range(6))
+@pytest.mark.parametrize("edge", range(7))
 def test_streamlines_match_the_oracle(ctx, port, edge):
     from pars_gb300 import native, workloads as W
     f = W.abc_field(17)
@@ -35,7 +36,7 @@ def test_streamlines_match_the_oracle(ctx, port, edge):
     ctx.release_field(h)
 
 
-@pytest.mark.parametrize("edge", range(6))
+@pytest.mark.parametrize("edge", range(7))
 def test_domain_matches_the_oracle(ctx, port, edge):
     from pars_gb300 import native, workloads as W
     f = W.abc_field(17)
