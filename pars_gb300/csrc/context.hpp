@@ -223,7 +223,7 @@ struct pars_gpu_context
                                           block_of_next, exits, exit_keys, exit_keys_sorted, exit_order,
                                           exit_order_sorted, counters, block_max, cub_temp, scan_input, tile_counts,
                                           tile_offsets, staging, boundary_positions, boundary_offsets, single_block,
-                                          slot_layouts, curve_bounds, color_specs;
+                                          slot_layouts, curve_bounds, color_specs, index_flags;
   pars::device_buffer                     ftle;
   long long                               ftle_count = 0;
   // asynchronous rounds: segment table, vertex chunks, round order

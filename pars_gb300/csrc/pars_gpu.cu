@@ -29,7 +29,7 @@ void for_each_scratch(context_type& c, visit_type&& visit)
                   &c.exit_order_sorted, &c.counters, &c.block_max, &c.cub_temp, &c.scan_input, &c.tile_counts,
                   &c.tile_offsets, &c.staging, &c.ftle, &c.curves.vertices, &c.curves.colors,
                   &c.curves.indices, &c.boundary_positions, &c.boundary_offsets, &c.batch_jobs,
-                  &c.batch_counters, &c.single_block, &c.slot_layouts, &c.curve_bounds, &c.color_specs})
+                  &c.batch_counters, &c.single_block, &c.slot_layouts, &c.curve_bounds, &c.color_specs, &c.index_flags})
     visit(*b);
 }
 }
