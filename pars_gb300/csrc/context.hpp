@@ -227,8 +227,8 @@ struct pars_gpu_context
   pars::device_buffer                     ftle;
   long long                               ftle_count = 0;
   // asynchronous rounds: segment table, vertex chunks, round order
-  pars::device_buffer                     async_segments, async_chunks, async_counters, async_order, async_positions,
-                                          async_cursor;
+  pars::device_buffer                     async_segments, async_chunks, async_counters, async_order,
+                                          async_rounds;
   // round-by-round tracing (pars_gpu_round_trace): the next round's
   // particles stay in particles_in / block_of; their per-block counts and
   // largest remaining_iterations, the round they belong to, and the tracing
@@ -383,15 +383,13 @@ void launch_async_seed(pars_gpu_context& ctx, const async_launch& a, const pars_
 // Histogram of segment rounds (rounds_cap bins) and the largest round.
 void launch_round_histogram(pars_gpu_context& ctx, const int* seg_round, long long count, int rounds_cap, int* histogram,
                             int* max_round);
-// Segment ids grouped by round: ids[first[r] + k] for the k-th segment of round r met (any order).
-void launch_round_scatter(pars_gpu_context& ctx, const int* seg_round, long long count, const long long* first, int* cursor,
-                          unsigned int* ids);
-// key[k] = (seg_block[ids[k]] << 40) | position[seg_parent[ids[k]]] for a round's segments (the
-// segment's own id for seeds).
-void launch_round_keys(pars_gpu_context& ctx, const unsigned int* ids, long long n, const int* seg_block, const long long* seg_parent,
-                       const long long* position, unsigned long long* keys);
-// position[ids[k]] = first + k.
-void launch_round_positions(pars_gpu_context& ctx, const unsigned int* ids, long long n, long long first, long long* position);
+constexpr unsigned int async_no_segment = 0xffffffffu;
+// child[s] = the segment that continues s (others are left as they are).
+void launch_round_children(pars_gpu_context& ctx, const long long* seg_parent, long long count, unsigned int* child);
+// A round's candidates in the order of their senders: ids[k] = child[previous[k]] (k where previous is
+// null) and its block, no_block where there is none.
+void launch_round_keys(pars_gpu_context& ctx, const unsigned int* previous, long long n, const unsigned int* child, const int* seg_block,
+                       unsigned int no_block, unsigned int* keys, unsigned int* ids);
 // Per (round, block): segments and largest remaining_iterations, stats[2 * (round * blocks + block) + {0, 1}];
 // kept_ordered[g] = seg_kept[order[g]].
 void launch_round_stats(pars_gpu_context& ctx, const unsigned int* order, long long n, const int* seg_round, const int* seg_block,

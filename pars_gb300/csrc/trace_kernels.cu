@@ -464,36 +464,27 @@ __global__ void round_histogram_kernel(const int* __restrict__ seg_round, long l
   if (valid && lane == __ffs(same) - 1 && r < rounds_cap) atomicAdd(histogram + r, __popc(same));
 }
 
-__global__ void round_scatter_kernel(const int* __restrict__ seg_round, long long count, const long long* __restrict__ first,
-                                     int* __restrict__ cursor, unsigned int* __restrict__ ids)
+// child[s]: the segment that continues segment s (each has at most one).
+__global__ void round_children_kernel(const long long* __restrict__ seg_parent, long long count, unsigned int* __restrict__ child)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  const bool valid = i < count;
-  const int r = valid ? seg_round[i] : -1;
-  const unsigned same = __match_any_sync(full_mask, r);
-  const int leader = __ffs(same) - 1;
-  int base = 0;
-  if (valid && lane == leader) base = atomicAdd(cursor + r, __popc(same));
-  base = __shfl_sync(full_mask, base, leader);
-  if (valid) ids[first[r] + base + __popc(same & ((1u << lane) - 1u))] = (unsigned int)i;
+  if (i >= count) return;
+  const long long parent = seg_parent[i];
+  if (parent >= 0) child[parent] = (unsigned int)i;
 }
 
-__global__ void round_keys_kernel(const unsigned int* __restrict__ ids, long long n, const int* __restrict__ seg_block,
-                                  const long long* __restrict__ seg_parent, const long long* __restrict__ position,
-                                  unsigned long long* __restrict__ keys)
+// The candidates of a round in the order of their senders, and their blocks:
+// the children of the previous round's segments (key no_block: none), or the
+// segments themselves where `previous` is null (round 0).
+__global__ void round_keys_kernel(const unsigned int* __restrict__ previous, long long n, const unsigned int* __restrict__ child,
+                                  const int* __restrict__ seg_block, unsigned int no_block, unsigned int* __restrict__ keys,
+                                  unsigned int* __restrict__ ids)
 {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
-  const unsigned int s = ids[k];
-  const long long parent = seg_parent[s];
-  keys[k] = ((unsigned long long)seg_block[s] << 40) | (unsigned long long)(parent < 0 ? (long long)s : position[parent]);
-}
-
-__global__ void round_positions_kernel(const unsigned int* __restrict__ ids, long long n, long long first, long long* __restrict__ position)
-{
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) position[ids[k]] = first + k;
+  const unsigned int s = previous ? child[previous[k]] : (unsigned int)k;
+  keys[k] = s == async_no_segment ? no_block : (unsigned int)seg_block[s];
+  ids[k] = s;
 }
 
 __global__ void round_stats_kernel(const unsigned int* __restrict__ order, long long n, const int* __restrict__ seg_round,
@@ -723,27 +714,19 @@ void launch_round_histogram(pars_gpu_context& ctx, const int* seg_round, long lo
   round_histogram_kernel<<<grid_for(count, 256), 256, 0, ctx.stream>>>(seg_round, count, rounds_cap, histogram, max_round);
 }
 
-void launch_round_scatter(pars_gpu_context& ctx, const int* seg_round, long long count, const long long* first, int* cursor,
-                          unsigned int* ids)
+void launch_round_children(pars_gpu_context& ctx, const long long* seg_parent, long long count, unsigned int* child)
 {
   if (count <= 0) return;
-  launch_scope scope(ctx, "round_scatter");
-  round_scatter_kernel<<<grid_for(count, 256), 256, 0, ctx.stream>>>(seg_round, count, first, cursor, ids);
+  launch_scope scope(ctx, "round_children");
+  round_children_kernel<<<grid_for(count, 256), 256, 0, ctx.stream>>>(seg_parent, count, child);
 }
 
-void launch_round_keys(pars_gpu_context& ctx, const unsigned int* ids, long long n, const int* seg_block, const long long* seg_parent,
-                       const long long* position, unsigned long long* keys)
+void launch_round_keys(pars_gpu_context& ctx, const unsigned int* previous, long long n, const unsigned int* child, const int* seg_block,
+                       unsigned int no_block, unsigned int* keys, unsigned int* ids)
 {
   if (n <= 0) return;
   launch_scope scope(ctx, "round_keys");
-  round_keys_kernel<<<grid_for(n, 256), 256, 0, ctx.stream>>>(ids, n, seg_block, seg_parent, position, keys);
-}
-
-void launch_round_positions(pars_gpu_context& ctx, const unsigned int* ids, long long n, long long first, long long* position)
-{
-  if (n <= 0) return;
-  launch_scope scope(ctx, "round_positions");
-  round_positions_kernel<<<grid_for(n, 256), 256, 0, ctx.stream>>>(ids, n, first, position);
+  round_keys_kernel<<<grid_for(n, 256), 256, 0, ctx.stream>>>(previous, n, child, seg_block, no_block, keys, ids);
 }
 
 void launch_round_stats(pars_gpu_context& ctx, const unsigned int* order, long long n, const int* seg_round, const int* seg_block,
