@@ -562,6 +562,40 @@ __global__ void __launch_bounds__(256) compact_kernel(const float4* __restrict__
   }
 }
 
+// out[0 .. count] = exclusive sums of in for at most scan_small values, by one CTA:
+// scan_items values a thread, warp scans, the warps' totals through shared memory.
+constexpr int scan_threads = 1024, scan_items = 8, scan_small = scan_threads * scan_items;
+__global__ void __launch_bounds__(scan_threads) scan_kernel(const int* __restrict__ in, long long* __restrict__ out, int count)
+{
+  __shared__ long long totals[scan_threads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first = threadIdx.x * scan_items;
+  int v[scan_items];
+  long long sum = 0;
+  #pragma unroll
+  for (int k = 0; k < scan_items; ++k) { v[k] = first + k < count ? in[first + k] : 0; sum += v[k]; }
+  long long at = sum;
+  #pragma unroll
+  for (int off = 1; off < 32; off <<= 1)
+  {
+    const long long o = __shfl_up_sync(full_mask, at, off);
+    if (lane >= off) at += o;
+  }
+  if (lane == 31) totals[warp] = at;
+  __syncthreads();
+  long long before = lane < warp ? totals[lane] : 0;
+  #pragma unroll
+  for (int off = 16; off; off >>= 1) before += __shfl_xor_sync(full_mask, before, off);
+  at += before - sum;
+  #pragma unroll
+  for (int k = 0; k < scan_items; ++k)
+  {
+    if (first + k < count) out[first + k] = at;
+    at += v[k];
+  }
+  if (threadIdx.x == scan_threads - 1) out[count] = at;
+}
+
 __global__ void widen_kernel(const int* __restrict__ in, long long* __restrict__ out, long long count)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -756,6 +790,15 @@ void launch_compact_vertices(pars_gpu_context& ctx, const float4* slots, const s
 
 void exclusive_sum(pars_gpu_context& ctx, const int* in, long long* out, long long count)
 {
+  // One launch instead of three while one CTA takes the values in one go (8000
+  // values: 10.6 us, 16.0 with the device-wide scan; 1000: 6.2, 15.4; two rounds,
+  // 16000: 15.9, 16.0).
+  if (count <= scan_small)
+  {
+    launch_scope scope(ctx, "scan");
+    scan_kernel<<<1, scan_threads, 0, ctx.stream>>>(in, out, (int)count);
+    return;
+  }
   // Widen to int64 with a trailing zero, so that the exclusive scan over
   // count + 1 entries leaves the total in out[count].
   ctx.scan_input.reserve(sizeof(long long) * (count + 1));

@@ -20,3 +20,11 @@ def test_indices_match_the_oracle(ctx, port, n):
         term[at[rng.random(len(at)) < 0.5] - 1] = True
     v[term] = (-2.0, -2.0, -2.0, 0.0)
     assert np.array_equal(ctx.index_generate(v), port.index_generate(v))
+
+
+@pytest.mark.parametrize("tiles", [1, 31, 33, 1023, 1025, 8191, 8192, 8193])
+def test_tile_offsets_of_one_and_of_many_blocks(ctx, tiles):
+    """Every vertex indexed but the last: the scan's offsets show in every index."""
+    n = tiles * 2048 - 5
+    v = np.ones((n, 4), np.float32)
+    assert np.array_equal(ctx.index_generate(v), np.arange(n - 1, dtype=np.int32))
