@@ -415,8 +415,10 @@ void launch_gather_exits(pars_gpu_context& ctx, const pars_particle* exits, cons
 void launch_iota(pars_gpu_context& ctx, unsigned int* out, long long count);
 // out[k] = offsets[positions[k]] for k < n.
 void launch_gather_offsets(pars_gpu_context& ctx, const long long* offsets, const long long* positions, long long n, long long* out);
-// block_max[0] = max remaining_iterations over particles (block_of == nullptr).
-void launch_particle_stats(pars_gpu_context& ctx, const pars_particle* particles, const int* block_of, long long count, int* block_max);
+// Each block's largest remaining_iterations and each particle's block (block_of, if given), for particles
+// grouped by block, block b from first[b] on (one block: first may be null).
+void launch_particle_stats(pars_gpu_context& ctx, const pars_particle* particles, const long long* first, int blocks, long long count,
+                           int* block_of, int* block_max);
 // Copies the ghosted block at voxel `offset` of a device [X][Y][Z][3] domain into float4 [shape].
 void launch_extract_block(pars_gpu_context& ctx, const float* domain_xyz, const int32_t domain[3], const int32_t offset[3],
                           const int shape[3], float4* out);

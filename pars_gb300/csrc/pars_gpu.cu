@@ -389,8 +389,8 @@ struct round_plan
   std::vector<int>       block_max;
 };
 
-// The tracing counters: steps (accumulated over rounds), the exit-queue size
-// (32-bit) and the tracing kernel's pool counter.
+// The tracing counters, one after the other: steps (accumulated over rounds), the
+// exit-queue size (32-bit) and the tracing kernel's pool counter.
 struct round_counters
 {
   unsigned long long* steps;
@@ -423,7 +423,7 @@ void clear_curves(pars_gpu_context& ctx)
 // particles in ctx.particles_in, and `plan` describes them.
 void trace_one_round(pars_gpu_context& ctx, const std::vector<trace_block>& blocks, const trace_block* device_blocks,
                      round_plan& plan, const step_rule& rule, bool route_exits, int round, const round_counters& counters,
-                     const step_rule* device_block_rules)
+                     const step_rule* device_block_rules, unsigned long long& steps)
 {
   auto& curves = ctx.curves;
   const int nblocks = int(blocks.size());
@@ -458,8 +458,7 @@ void trace_one_round(pars_gpu_context& ctx, const std::vector<trace_block>& bloc
     ctx.exits.reserve(sizeof(pars_particle) * count);
     ctx.exit_keys.reserve(sizeof(unsigned long long) * count);
   }
-  PARS_CUDA(cudaMemsetAsync(counters.exits, 0, sizeof(unsigned int), ctx.stream));
-  PARS_CUDA(cudaMemsetAsync(counters.pool, 0, sizeof(unsigned long long), ctx.stream));
+  PARS_CUDA(cudaMemsetAsync(counters.exits, 0, 2 * sizeof(unsigned long long), ctx.stream));   // and the pool counter
 
   trace_launch a {};
   a.blocks = device_blocks;
@@ -499,20 +498,30 @@ void trace_one_round(pars_gpu_context& ctx, const std::vector<trace_block>& bloc
       pending.push_back({first + std::min(n, k * ppc), first + std::min(n, (k + 1) * ppc), b});
     first += n;
   }
+  struct { unsigned long long steps; unsigned int exits, padding; } read {};
+  std::vector<long long> boundary(pending.size() * 2 + 1, 0);
   std::vector<long long> positions;
-  positions.reserve(pending.size() * 2 + 1);
-  for (auto& p : pending) { positions.push_back(p.first); positions.push_back(p.last); }
-  positions.push_back(count);
-  std::vector<long long> boundary(positions.size());
-  ctx.boundary_positions.reserve(sizeof(long long) * positions.size());
-  ctx.boundary_offsets.reserve(sizeof(long long) * positions.size());
-  PARS_CUDA(cudaMemcpyAsync(ctx.boundary_positions.get(), positions.data(), sizeof(long long) * positions.size(), cudaMemcpyHostToDevice, ctx.stream));
-  launch_gather_offsets(ctx, ctx.offsets.as<const long long>(), ctx.boundary_positions.as<const long long>(), (long long)positions.size(),
-                        ctx.boundary_offsets.as<long long>());
-  unsigned int exit_total = 0;
-  PARS_CUDA(cudaMemcpyAsync(boundary.data(), ctx.boundary_offsets.get(), sizeof(long long) * boundary.size(), cudaMemcpyDeviceToHost, ctx.stream));
-  PARS_CUDA(cudaMemcpyAsync(&exit_total, counters.exits, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx.stream));
+  if (pending.size() == 1)
+  {
+    // one batch: from 0 to the total
+    PARS_CUDA(cudaMemcpyAsync(&boundary.back(), ctx.offsets.as<long long>() + count, sizeof(long long), cudaMemcpyDeviceToHost, ctx.stream));
+  }
+  else
+  {
+    positions.reserve(boundary.size());
+    for (auto& p : pending) { positions.push_back(p.first); positions.push_back(p.last); }
+    positions.push_back(count);
+    ctx.boundary_positions.reserve(sizeof(long long) * positions.size());
+    ctx.boundary_offsets.reserve(sizeof(long long) * positions.size());
+    PARS_CUDA(cudaMemcpyAsync(ctx.boundary_positions.get(), positions.data(), sizeof(long long) * positions.size(), cudaMemcpyHostToDevice, ctx.stream));
+    launch_gather_offsets(ctx, ctx.offsets.as<const long long>(), ctx.boundary_positions.as<const long long>(), (long long)positions.size(),
+                          ctx.boundary_offsets.as<long long>());
+    PARS_CUDA(cudaMemcpyAsync(boundary.data(), ctx.boundary_offsets.get(), sizeof(long long) * boundary.size(), cudaMemcpyDeviceToHost, ctx.stream));
+  }
+  PARS_CUDA(cudaMemcpyAsync(&read, counters.steps, sizeof(read), cudaMemcpyDeviceToHost, ctx.stream));
   PARS_CUDA(cudaStreamSynchronize(ctx.stream));
+  if (pending.size() == 1) boundary[1] = boundary[2];
+  steps = read.steps;
   const long long round_vertices = boundary.back();
 
   grow_curves(ctx, curves.vertex_total + round_vertices);
@@ -532,7 +541,7 @@ void trace_one_round(pars_gpu_context& ctx, const std::vector<trace_block>& bloc
 
   // Exchange: the exit queue, stably ordered by (destination block, source
   // order), becomes the next round's particle list.
-  const long long next = route_exits ? (long long)exit_total : 0;
+  const long long next = route_exits ? (long long)read.exits : 0;
   std::fill(block_count.begin(), block_count.end(), 0);
   std::fill(block_max.begin(), block_max.end(), 0);
   if (next > 0)
@@ -577,14 +586,13 @@ void run_rounds(pars_gpu_context& ctx, const std::vector<trace_block>& blocks, c
   plan.block_count = std::move(block_count);
   plan.block_max = std::move(block_max);
   int round = 0;
+  unsigned long long steps = 0;
   while (plan.count > 0)
   {
-    trace_one_round(ctx, blocks, device_blocks, plan, rule, route_exits, round, counters, device_block_rules);
+    trace_one_round(ctx, blocks, device_blocks, plan, rule, route_exits, round, counters, device_block_rules, steps);
     ++round;
   }
 
-  unsigned long long steps = 0;
-  PARS_CUDA(cudaMemcpyAsync(&steps, counters.steps, sizeof(steps), cudaMemcpyDeviceToHost, ctx.stream));
   PARS_CUDA(cudaStreamSynchronize(ctx.stream));
   if (summary)
   {
@@ -679,18 +687,23 @@ bool run_rounds_async(pars_gpu_context& ctx, const std::vector<trace_block>& blo
   // 350 k segments in all took 640 us, now 250.
   constexpr int rounds_cap = 65536;
   ctx.async_rounds.reserve(sizeof(int) * (rounds_cap + 1));
-  int* histogram = ctx.async_rounds.as<int>();
-  int* max_round = histogram + rounds_cap;
-  PARS_CUDA(cudaMemsetAsync(histogram, 0, sizeof(int) * (rounds_cap + 1), ctx.stream));
+  int* max_round = ctx.async_rounds.as<int>();
+  int* histogram = max_round + 1;
+  PARS_CUDA(cudaMemsetAsync(max_round, 0, sizeof(int) * (rounds_cap + 1), ctx.stream));
   launch_round_histogram(ctx, a.seg_round, n, rounds_cap, histogram, max_round);
-  int rounds = 0;
-  PARS_CUDA(cudaMemcpyAsync(&rounds, max_round, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+  constexpr int read_rounds = 255;   // with max_round in one read; more take a second
+  std::vector<int> per_round(1 + read_rounds);
+  PARS_CUDA(cudaMemcpyAsync(per_round.data(), max_round, sizeof(int) * per_round.size(), cudaMemcpyDeviceToHost, ctx.stream));
   PARS_CUDA(cudaStreamSynchronize(ctx.stream));
-  ++rounds;
+  const int rounds = per_round[0] + 1;
   if (rounds > rounds_cap) return false;
-  std::vector<int> per_round(rounds);
-  PARS_CUDA(cudaMemcpyAsync(per_round.data(), histogram, sizeof(int) * rounds, cudaMemcpyDeviceToHost, ctx.stream));
-  PARS_CUDA(cudaStreamSynchronize(ctx.stream));
+  per_round.erase(per_round.begin());
+  per_round.resize(rounds);
+  if (rounds > read_rounds)
+  {
+    PARS_CUDA(cudaMemcpyAsync(per_round.data(), histogram, sizeof(int) * rounds, cudaMemcpyDeviceToHost, ctx.stream));
+    PARS_CUDA(cudaStreamSynchronize(ctx.stream));
+  }
   std::vector<long long> first(rounds + 1, 0);
   long long widest = 0;
   for (int r = 0; r < rounds; ++r) { first[r + 1] = first[r] + per_round[r]; widest = std::max<long long>(widest, per_round[r]); }
@@ -802,8 +815,9 @@ const trace_block* single_block(pars_gpu_context& ctx, field_entry& f, std::vect
   return ctx.single_block.as<const trace_block>();
 }
 
-void trace_single(pars_gpu_context& ctx, int32_t field, long long count, int32_t integrator, int32_t stage_mode,
-                  float step_size, pars_gpu_trace_summary* summary)
+// `host`: the particles in host memory, if that is where they came from.
+void trace_single(pars_gpu_context& ctx, int32_t field, long long count, const pars_particle* host, int32_t integrator,
+                  int32_t stage_mode, float step_size, pars_gpu_trace_summary* summary)
 {
   auto& f = find_field(ctx, field);
   const step_rule rule = make_rule(integrator, stage_mode, step_size);
@@ -811,11 +825,15 @@ void trace_single(pars_gpu_context& ctx, int32_t field, long long count, int32_t
   const trace_block* device_blocks = single_block(ctx, f, blocks);
   std::vector<long long> block_count(1, count);
   std::vector<int> block_max(1, 0);
-  if (count > 0)
+  // The largest remaining_iterations: a few host particles are read faster than a
+  // kernel's answer comes back (about 25 us; 32768 particles take about as long).
+  if (host && count <= 32768)
+    for (long long i = 0; i < count; ++i) block_max[0] = std::max(block_max[0], host[i].remaining_iterations);
+  else if (count > 0)
   {
     ctx.block_max.reserve(sizeof(int) * 2);
     PARS_CUDA(cudaMemsetAsync(ctx.block_max.get(), 0, sizeof(int) * 2, ctx.stream));
-    launch_particle_stats(ctx, ctx.particles_in.as<const pars_particle>(), nullptr, count, ctx.block_max.as<int>());
+    launch_particle_stats(ctx, ctx.particles_in.as<const pars_particle>(), nullptr, 1, count, nullptr, ctx.block_max.as<int>());
     PARS_CUDA(cudaMemcpyAsync(block_max.data(), ctx.block_max.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
     PARS_CUDA(cudaStreamSynchronize(ctx.stream));
   }
@@ -1529,7 +1547,7 @@ int32_t pars_gpu_trace(pars_gpu_context* ctx, int32_t field, const pars_particle
     ctx->particles_in.reserve(checked_bytes(std::max<long long>(count, 1), sizeof(pars_particle)));
     if (count > 0)
       PARS_CUDA(cudaMemcpyAsync(ctx->particles_in.get(), particles, sizeof(pars_particle) * count, cudaMemcpyHostToDevice, ctx->stream));
-    trace_single(*ctx, field, count, integrator, stage_mode, step_size, summary);
+    trace_single(*ctx, field, count, particles, integrator, stage_mode, step_size, summary);
   });
 }
 
@@ -1541,7 +1559,7 @@ int32_t pars_gpu_trace_device(pars_gpu_context* ctx, int32_t field, const pars_p
     ctx->particles_in.reserve(checked_bytes(std::max<long long>(count, 1), sizeof(pars_particle)));
     if (count > 0)
       PARS_CUDA(cudaMemcpyAsync(ctx->particles_in.get(), device_particles, sizeof(pars_particle) * count, cudaMemcpyDeviceToDevice, ctx->stream));
-    trace_single(*ctx, field, count, integrator, stage_mode, step_size, summary);
+    trace_single(*ctx, field, count, nullptr, integrator, stage_mode, step_size, summary);
   });
 }
 
@@ -1640,26 +1658,28 @@ int32_t pars_gpu_trace_domain(pars_gpu_context* ctx, int32_t domain, const pars_
     const int nblocks = d.ranks;
     const long long count = seed_offsets[nblocks] - seed_offsets[0];
     PARS_REQUIRE(count >= 0 && (count == 0 || particles), "particles are required");
-    std::vector<long long> block_count(nblocks);
+    std::vector<long long> block_count(nblocks), first(nblocks + 1, 0);
     std::vector<int> block_max(nblocks, 0);
-    std::vector<int> block_of(std::max<long long>(count, 1));
     for (int b = 0; b < nblocks; ++b)
     {
-      const long long begin = seed_offsets[b] - seed_offsets[0], end = seed_offsets[b + 1] - seed_offsets[0];
-      PARS_REQUIRE(end >= begin, "seed_offsets must be non-decreasing");
-      block_count[b] = end - begin;
-      for (long long i = begin; i < end; ++i)
-      {
-        block_of[i] = b;
-        block_max[b] = std::max(block_max[b], particles[seed_offsets[0] + i].remaining_iterations);
-      }
+      PARS_REQUIRE(seed_offsets[b + 1] >= seed_offsets[b], "seed_offsets must be non-decreasing");
+      block_count[b] = seed_offsets[b + 1] - seed_offsets[b];
+      first[b + 1] = first[b] + block_count[b];
     }
     ctx->particles_in.reserve(checked_bytes(std::max<long long>(count, 1), sizeof(pars_particle)));
     ctx->block_of.reserve(checked_bytes(std::max<long long>(count, 1), sizeof(int)));
     if (count > 0)
     {
+      // each particle's block and the blocks' largest remaining_iterations, on the device
+      ctx->boundary_positions.reserve(sizeof(long long) * (nblocks + 1));
+      ctx->block_max.reserve(sizeof(int) * 2 * nblocks);
       PARS_CUDA(cudaMemcpyAsync(ctx->particles_in.get(), particles + seed_offsets[0], sizeof(pars_particle) * count, cudaMemcpyHostToDevice, ctx->stream));
-      PARS_CUDA(cudaMemcpyAsync(ctx->block_of.get(), block_of.data(), sizeof(int) * count, cudaMemcpyHostToDevice, ctx->stream));
+      PARS_CUDA(cudaMemcpyAsync(ctx->boundary_positions.get(), first.data(), sizeof(long long) * (nblocks + 1), cudaMemcpyHostToDevice, ctx->stream));
+      PARS_CUDA(cudaMemsetAsync(ctx->block_max.get(), 0, sizeof(int) * nblocks, ctx->stream));
+      launch_particle_stats(*ctx, ctx->particles_in.as<const pars_particle>(), ctx->boundary_positions.as<const long long>(), nblocks, count,
+                            ctx->block_of.as<int>(), ctx->block_max.as<int>());
+      PARS_CUDA(cudaMemcpyAsync(block_max.data(), ctx->block_max.get(), sizeof(int) * nblocks, cudaMemcpyDeviceToHost, ctx->stream));
+      PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     }
     // one persistent launch over all rounds; round by round when its
     // buffers do not fit or overflow
@@ -1759,12 +1779,11 @@ int32_t pars_gpu_round_trace(pars_gpu_context* ctx, int32_t domain, int32_t roun
     const long long vertices_before = ctx->curves.vertex_total;
     const round_counters counters = tracing_counters(*ctx);
     PARS_CUDA(cudaMemsetAsync(counters.steps, 0, sizeof(unsigned long long), ctx->stream));
+    unsigned long long steps = 0;
     if (plan.count > 0)
-      trace_one_round(*ctx, d.blocks, d.device_blocks.as<const trace_block>(), plan, rule, true, round, counters, nullptr);
+      trace_one_round(*ctx, d.blocks, d.device_blocks.as<const trace_block>(), plan, rule, true, round, counters, nullptr, steps);
     else
       std::fill(plan.block_count.begin(), plan.block_count.end(), 0);
-    unsigned long long steps = 0;
-    PARS_CUDA(cudaMemcpyAsync(&steps, counters.steps, sizeof(steps), cudaMemcpyDeviceToHost, ctx->stream));
     PARS_CUDA(cudaStreamSynchronize(ctx->stream));
     ctx->round_serial = ctx->trace_serial;
     ctx->round_domain = domain;

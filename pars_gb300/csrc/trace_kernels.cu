@@ -631,13 +631,31 @@ __global__ void gather_offsets_kernel(const long long* __restrict__ offsets, con
   if (k < n) out[k] = offsets[positions[k]];
 }
 
-__global__ void particle_stats_kernel(const pars_particle* __restrict__ particles, const int* __restrict__ block_of, long long count,
-                                      int* __restrict__ block_max)
+// Each block's largest remaining_iterations, and each particle's block (block_of, if
+// given), for particles grouped by block: block b's are first[b] .. first[b + 1] - 1
+// (one block: `first` is not read).  A warp's particles are mostly of one block, so
+// it takes one atomic per block it meets.
+__global__ void particle_stats_kernel(const pars_particle* __restrict__ particles, const long long* __restrict__ first, int blocks,
+                                      long long count, int* __restrict__ block_of, int* __restrict__ block_max)
 {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int block = block_of ? block_of[i] : 0;
-  atomicMax(block_max + block, particles[i].remaining_iterations);
+  int block = -1, remaining = 0;
+  if (i < count)
+  {
+    int lo = 0, hi = blocks - 1;
+    while (lo < hi)
+    {
+      const int mid = (lo + hi + 1) >> 1;
+      if (first[mid] <= i) lo = mid;
+      else hi = mid - 1;
+    }
+    block = lo;
+    if (block_of) block_of[i] = block;
+    remaining = particles[i].remaining_iterations;
+  }
+  const unsigned same = __match_any_sync(full_mask, block);
+  const int top = __reduce_max_sync(same, remaining);
+  if (block >= 0 && int(threadIdx.x & 31) == __ffs(same) - 1) atomicMax(block_max + block, top);
 }
 
 __global__ void extract_block_kernel(const float* __restrict__ domain, int dy, int dz, int ox, int oy, int oz,
@@ -864,11 +882,12 @@ void launch_gather_offsets(pars_gpu_context& ctx, const long long* offsets, cons
   gather_offsets_kernel<<<grid_for(n, 256), 256, 0, ctx.stream>>>(offsets, positions, n, out);
 }
 
-void launch_particle_stats(pars_gpu_context& ctx, const pars_particle* particles, const int* block_of, long long count, int* block_max)
+void launch_particle_stats(pars_gpu_context& ctx, const pars_particle* particles, const long long* first, int blocks, long long count,
+                           int* block_of, int* block_max)
 {
   if (count <= 0) return;
   launch_scope scope(ctx, "particle_stats");
-  particle_stats_kernel<<<grid_for(count, 256), 256, 0, ctx.stream>>>(particles, block_of, count, block_max);
+  particle_stats_kernel<<<grid_for(count, 256), 256, 0, ctx.stream>>>(particles, first, blocks, count, block_of, block_max);
 }
 
 void launch_extract_block(pars_gpu_context& ctx, const float* domain_xyz, const int32_t domain[3], const int32_t offset[3],
