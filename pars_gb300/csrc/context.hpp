@@ -326,6 +326,7 @@ struct trace_launch
   const pars_particle* particles;
   const int*           block_of;      // nullptr: every particle is in block 0
   long long            count;
+  long long            field_bytes;   // of the largest block
   const slot_layout*   block_slots;   // per block (device)
   float4*              slots;
   int*                 written;

@@ -819,9 +819,35 @@ __device__ __forceinline__ bool is_zero_local(const field_view& f, const float3&
   return fabsf(v.x) <= 1e-5f * f.inv_hx && fabsf(v.y) <= 1e-5f * f.inv_hy && fabsf(v.z) <= 1e-5f * f.inv_hz;
 }
 
-// One classical RK4 (or Euler) step in local coordinates with k1 sampled at q.
-__device__ __forceinline__ void local_step(const field_view& f, corner_cache& k, int rk4, float h, local_position& q, const float3& k1)
+// Starts the copies that bring the corners of the cell at offset (wx, wy, wz) from
+// q's cell into L1, unless k holds them.  Asynchronous copies to shared memory
+// (`slot`, 16 bytes that nobody reads) need no register that a later instruction
+// would wait for.
+__device__ __forceinline__ void fetch_cell(const field_view& f, const corner_cache& k, const local_position& q, float wx, float wy, float wz,
+                                           unsigned int slot)
 {
+  if (in_unit_cube(wx, wy, wz)) return;
+  int ix = q.ix, iy = q.iy, iz = q.iz;
+  find_cell(f, ix, iy, iz, wx, wy, wz);
+  if (ix == k.ix && iy == k.iy && iz == k.iz) return;
+  const long long syz = (long long)f.ny * f.nz;
+  const float4* base = f.data + ((long long)ix * f.ny + iy) * f.nz + iz;
+  #pragma unroll
+  for (int c = 0; c < 8; ++c)
+  {
+    const float4* corner = base + (c & 4 ? syz : 0) + (c & 2 ? f.nz : 0) + (c & 1);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"(slot), "l"(corner));
+  }
+}
+
+// One classical RK4 (or Euler) step in local coordinates with k1 sampled at q.
+// FETCH: the cell where the step is expected to end is fetched into L1 while the
+// stages before it are sampled (`slot`: see fetch_cell).
+template <bool FETCH = false>
+__device__ __forceinline__ void local_step(const field_view& f, corner_cache& k, int rk4, float h, local_position& q, const float3& k1,
+                                           unsigned int slot = 0)
+{
+  if constexpr (FETCH) fetch_cell(f, k, q, fmaf(h, k1.x, q.ux), fmaf(h, k1.y, q.uy), fmaf(h, k1.z, q.uz), slot);
   if (!rk4)
   {
     compensated_add(q.ux, q.lx, h * k1.x);

@@ -465,6 +465,8 @@ void trace_one_round(pars_gpu_context& ctx, const std::vector<trace_block>& bloc
   a.particles = ctx.particles_in.as<const pars_particle>();
   a.block_of = nblocks > 1 ? ctx.block_of.as<const int>() : nullptr;
   a.count = count;
+  for (const trace_block& b : blocks)
+    a.field_bytes = std::max(a.field_bytes, (long long)sizeof(float4) * b.field.nx * b.field.ny * b.field.nz);
   a.block_slots = ctx.slot_layouts.as<const slot_layout>();
   a.slots = ctx.slots.as<float4>();
   a.written = ctx.written.as<int>();

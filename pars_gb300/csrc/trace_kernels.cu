@@ -74,8 +74,8 @@ enum iteration_outcome { particle_stepped = 0, particle_ended = 1, particle_left
 // The per-particle part of one iteration: the termination tests and the step,
 // the vertex written at slot p.it.  particle_left: the step-start point is
 // outside the block (the caller routes the particle).
-template <int MODE>
-__device__ __forceinline__ int particle_advance(lane_particle& p, unsigned int& steps)
+template <int MODE, bool FETCH = false>
+__device__ __forceinline__ int particle_advance(lane_particle& p, unsigned int& steps, unsigned int slot = 0)
 {
   const float4 term = termination_vertex();
   if (p.it >= p.N) return particle_ended;                              // remaining_iterations <= 1
@@ -95,7 +95,7 @@ __device__ __forceinline__ int particle_advance(lane_particle& p, unsigned int& 
   else
   {
     if constexpr (MODE == trace_general) general_step_local(p.f, p.cache, p.rule, p.q, v, p.hist);
-    else local_step(p.f, p.cache, p.rule.rk4, p.rule.h, p.q, v);
+    else local_step<FETCH>(p.f, p.cache, p.rule.rk4, p.rule.h, p.q, v, slot);
     next = to_absolute(p.f, p.q, p.last.w);
   }
   p.out[p.it] = next;
@@ -133,10 +133,10 @@ __device__ __forceinline__ pars_particle handed_over(const lane_particle& p)
 // contains() only within an ulp of the block's last face), each vertex
 // written as offset + (cell + u) h.  MODE trace_general: the same for any
 // re-sampled scheme (general_step_local).
-template <int MODE>
-__device__ __forceinline__ bool particle_iteration(const trace_launch& a, lane_particle& p, unsigned int& steps)
+template <int MODE, bool FETCH = false>
+__device__ __forceinline__ bool particle_iteration(const trace_launch& a, lane_particle& p, unsigned int& steps, unsigned int slot = 0)
 {
-  const int outcome = particle_advance<MODE>(p, steps);
+  const int outcome = particle_advance<MODE, FETCH>(p, steps, slot);
   if (outcome == particle_stepped) return false;
   if (outcome == particle_left && a.route_exits)
   {
@@ -163,17 +163,27 @@ __device__ __forceinline__ void add_steps(const trace_launch& a, unsigned int st
 // One particle per thread, `lanes` of a warp's threads used: for launches with no
 // more particles than resident lanes, where refilling cannot help and warp votes
 // would only add latency.
-template <int MODE>
+// FETCH (re-sampled RK4 on fields that do not stay in L2): a step's stages lie in
+// other cells, and each waits for its corners before the next is known; the end
+// cell's are fetched while the middle ones are sampled.
+template <int MODE, bool FETCH = false>
 __global__ void __launch_bounds__(32) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
 {
+  unsigned int slot = 0;
+  if constexpr (FETCH)
+  {
+    __shared__ float4 slots[32];
+    slot = (unsigned int)__cvta_generic_to_shared(slots + threadIdx.x);
+  }
   const long long i = (long long)blockIdx.x * lanes + threadIdx.x;
   unsigned int steps = 0;
   if (int(threadIdx.x) < lanes && i < a.count)
   {
     lane_particle p;
     particle_start<MODE>(a, p, i);
-    while (!particle_iteration<MODE>(a, p, steps)) {}
+    while (!particle_iteration<MODE, FETCH>(a, p, steps, slot)) {}
   }
+  if constexpr (FETCH) asm volatile("cp.async.wait_all;" ::: "memory");
   add_steps(a, steps);
 }
 
@@ -716,7 +726,15 @@ void launch_trace(pars_gpu_context& ctx, const trace_launch& a)
     const int lanes = narrow_lanes(a.count, sms);
     const unsigned grid = (unsigned)((a.count + lanes - 1) / lanes);
     if (mode == trace_frozen)       trace_kernel<trace_frozen><<<grid, 32, 0, ctx.stream>>>(a, lanes);
-    else if (mode == trace_classic) trace_kernel<trace_classic><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    else if (mode == trace_classic)
+    {
+      // 10648 particles, 1000 RK4 steps on a 124 MB field: 1622 us, 1448 with the
+      // fetches; 12167 of 800 on 575 MB: 1029, 896; on 45 MB: 697, 671 (another flow:
+      // 743, 742); 4096 on 4 MB: 481, 495 (the corners are in L2, the fetches only cost
+      // issue).  Pools with every SM full lose: 117649 on 124 MB 1120, 1475.
+      if (a.rule.rk4 && a.field_bytes > (32LL << 20)) trace_kernel<trace_classic, true><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+      else trace_kernel<trace_classic><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    }
     else                            trace_kernel<trace_general><<<grid, 32, 0, ctx.stream>>>(a, lanes);
     return;
   }

@@ -54,3 +54,21 @@ def test_domain_matches_the_oracle(ctx, port, edge):
     assert s["steps"] == expected.steps
     compare(gpu_curves(ctx, s, "rgb"), expected.batches)
     ctx.domain_release(d)
+
+
+@pytest.mark.parametrize("n", [5, 700])
+def test_curves_on_a_large_field_do_not_depend_on_the_launch(ctx, n):
+    """Re-sampled RK4 on a field of more than 32 MB fetches cells ahead in a launch of few
+    particles; beside many others the same particles go through another kernel."""
+    from pars_gb300 import native, workloads as W
+    f = W.abc_field(132)
+    h = ctx.upload_field(f)
+    few = _seeds(native.PARTICLE_DTYPE, n, 40)
+    few["position"][: n // 2, :3] *= np.float32(0.02)   # near the faces: cells clamped, curves that leave
+    filler = _seeds(native.PARTICLE_DTYPE, 300000, 2)
+    curves = []
+    for p in (few, np.concatenate([few, filler])):
+        s = ctx.trace(h, p, 2, 1, 0.2)
+        curves.append(ctx.curves(s["batches"], vertices=True)[0]["vertices"])
+    assert np.array_equal(curves[0], curves[1][: len(curves[0])])
+    ctx.release_field(h)
