@@ -188,11 +188,12 @@ __global__ void __launch_bounds__(32) trace_kernel(const __grid_constant__ trace
 }
 
 // Persistent: warps take pools of particles from a device counter, and a lane
-// whose particle has ended takes the next particle of the pool at once (warp
-// ballot + prefix), so lanes do not idle while the rest of the warp finishes
-// longer curves.  Every particle writes only its own slot range, its counts
+// whose particle has ended takes the next particle of the pool (warp ballot +
+// prefix, after every pool_steps steps), so lanes do not idle while the rest of
+// the warp finishes longer curves.  Every particle writes only its own slot range, its counts
 // and its exit-queue entry, so the result does not depend on which lane traced
 // it.
+constexpr int pool_steps = 8;
 template <int MODE>
 __global__ void __launch_bounds__(128) trace_persistent_kernel(const __grid_constant__ trace_launch a, int pool_size)
 {
@@ -227,7 +228,9 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(const __grid_cons
       }
     }
     if (need == full_mask) break;   // every lane idle, and the pools are exhausted
-    if (alive && particle_iteration<MODE>(a, p, steps)) alive = false;
+    // (a look at the other lanes after every step: 991 against 784 us for 117649 frozen
+    // curves of 300 steps on 124 MB; re-sampled ones and 16 steps: within 2 %)
+    for (int k = 0; k < pool_steps && alive; ++k) alive = !particle_iteration<MODE>(a, p, steps);
   }
   add_steps(a, steps);
 }
