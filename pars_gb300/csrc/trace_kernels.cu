@@ -245,13 +245,18 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(const __grid_cons
 // every allocated segment is done (done read before allocated: a segment is
 // marked done only after its continuation was allocated and published).
 // What bounds the launch is its longest particle and every trip to L2 in its way:
-// lanes without a segment look for one every async_look turns only, and a warp with
-// nothing to trace polls less and less often (up to async_sleep ns apart), because
-// thousands of idle warps polling one counter slow every trip of the others.
-// 256^3 ABC in 64 blocks, re-sampled / frozen: 10 k seeds 4612 / 4403 us with a look
-// at every turn and polls 256 ns apart, 1525 / 1145 so; 100 k seeds 5963 / 5841,
-// 2285 / 1914; 512^3, 1 M seeds, the whole call: 22.8 ms, 19.1.
-constexpr int async_look = 16;
+// lanes take async_ahead steps between two looks at the warp (for segments, chunks
+// and the end: a dozen votes and trips to L2), and a warp with nothing to trace
+// polls less and less often (up to async_sleep ns apart), because thousands of idle
+// warps polling one counter slow every trip of the others.  256^3 ABC in 64 blocks,
+// re-sampled / frozen, 10 k and 100 k seeds:
+//   a look every step, polls 256 ns apart   4612 / 4403   5963 / 5841 us
+//   a look for segments every 16th step     1525 / 1145   2285 / 1914
+//   16 steps between looks                  1223 /  928   1795 / 1383
+//   (8 steps                                1234 /  959   1880 / 1581
+//    32 steps                               1244 /  945   1810 / 1290)
+// 512^3, 1 M seeds, the whole call: 22.8, 19.1, 12.5 ms.
+constexpr int async_ahead = 16;
 constexpr unsigned int async_sleep = 8192;
 constexpr unsigned int async_wait_limit = 1u << 20;   // warp-wide idle polls (about 10 s with the pauses)
 
@@ -312,7 +317,6 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
   long long pool_next = 0, pool_end = 0;       // warp-uniform: claimed ids not yet handed out
   long long slab_next = 0, slab_end = 0;       // warp-uniform: chunks not yet handed out
   int chunk = -1;
-  int turn = 0;
   lane_particle p;
   for (;;)
   {
@@ -336,14 +340,12 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
       if (k > left) { pool_next = fresh + (k - left); pool_end = fresh + a.lanes; }
       else pool_next += k;
     }
-    // Start a claimed segment once published: the seeds are from the start, a
-    // continuation is looked for every async_look turns while other lanes of the
-    // warp trace (a look is two trips to L2, which those lanes would wait for at
-    // every step).  Finish when every segment is done (done read before
+    // Start a claimed segment once published (the seeds are from the start; a look
+    // for another is two trips to L2).  Finish when every segment is done (done read before
     // allocated: equal counts mean nothing is in flight); that matters only to a
     // warp with nothing to trace.
     const bool idle = !__any_sync(full_mask, alive);
-    if (claim >= 0 && (claim < a.seeds || idle || turn % async_look == 0))
+    if (claim >= 0)
     {
       bool published = claim < a.seeds;
       if (!published && claim < a.capacity)
@@ -367,7 +369,6 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
         claim = -1;
       }
     }
-    ++turn;
     if (__all_sync(full_mask, finished)) break;
     if (!__any_sync(full_mask, alive))
     {
@@ -417,9 +418,14 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
       p.written = 1;
       p.kept = is_invalid_vertex(p.last) ? 0 : 1;
       p.it = 1;
-      continue;
     }
-    const int outcome = particle_advance<MODE>(p, steps);
+    // a few steps without a look at the other lanes, as far as the chunk goes
+    int outcome = particle_stepped;
+    for (int k = 0; k < async_ahead && outcome == particle_stepped; ++k)
+    {
+      outcome = particle_advance<MODE>(p, steps);
+      if (p.written % async_chunk == 0) break;
+    }
     if (outcome == particle_stepped) continue;
     if (outcome == particle_left)
     {
