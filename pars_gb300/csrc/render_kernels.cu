@@ -39,6 +39,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace pars
 {
@@ -630,6 +631,29 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   return r;
 }
 
+// The pixels of a rectangle that the segment's surroundings can touch: w pixels of
+// each row from ceil(base + slope row) on (of each column, the other way round, where
+// the segment is flatter than steep).  A point within `reach` of the segment is
+// within reach sqrt(1 + slope^2) of its line, measured along the row.
+struct screen_band
+{
+  int   columns, w;
+  float slope, base;
+};
+__device__ __forceinline__ screen_band band_of(const screen_rect& r)
+{
+  screen_band band {0, r.w, 0.0f, 0.0f};               // the whole rectangle
+  const bool flat = fabsf(r.along.x) > fabsf(r.along.y);
+  const float major = flat ? r.along.x : r.along.y, minor = flat ? r.along.y : r.along.x;
+  if (!(fabsf(major) > 1.0f) || r.radius2 == INFINITY) return band;
+  const float slope = __fdividef(minor, major);
+  const float half = sqrtf(r.radius2 * (1.0f + slope * slope)) + 0.01f;
+  if (!(half < 1024.0f)) return band;
+  const int w = int(2.0f * half) + 1;
+  if (w * (flat ? r.w : r.h) >= r.w * r.h) return band;
+  return screen_band {flat ? 1 : 0, w, slope, (flat ? r.from.y : r.from.x) - slope * (flat ? r.from.x : r.from.y) - half};
+}
+
 constexpr int raster_threads = 256;
 
 // The rectangles' pixels, all together and of the largest one.
@@ -706,7 +730,14 @@ __global__ void __launch_bounds__(256) raster_begin_kernel(const __grid_constant
 // the rectangles that start in it.  Pixels too far from the projected segment, or
 // already hit nearer, are dropped; the others are queued, and tested 32 at a
 // time, so that the capsule test runs with full warps.
-__global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_constant__ raster_args A)
+// Warps whose capsules cover more than 16 pixels walk the bands along the segments
+// (band_of) and take two turns at a time, so that the pixels' keys, which come from
+// L2, are waited for once.  10.6 M capsules on 1080 x 1920: 768 -> 669 us; long ones
+// (1.3 M from inside the flow) 1249 -> 882; bands with one turn at a time 711,
+// rectangles with two 758; tiny capsules (26.5 M on 960 x 540) do best with
+// rectangles and single turns: 407 us, 446 through the bands.  Limited by the keys'
+// latency at 32 warps per SM (64 registers; 48 registers 738, 72 registers 892).
+__global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_constant__ raster_args A)
 {
   if (!raster_applies(A, A.count)) return;
   struct __align__(16) entry
@@ -714,7 +745,11 @@ __global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_con
     float4 a, b;             // the segment; w: its start vertex, the nearest t
     float4 line;             // from, along
     float  inverse_length2, radius2, inverse_w;
-    int    w, x0, y0, start, padding;
+    int    w;                // pixels per row (or column) of the band
+    int    start, pixel;     // the rectangle's first pixel in the turns' order and on the screen
+    // bands only
+    int    across, columns;  // the rectangle's extent across the band; 1: the band is walked by columns
+    float  slope, base, padding[2];
   };
   __shared__ entry entries[raster_threads / 32][32];
   __shared__ uint2 queues[raster_threads / 32][64];
@@ -734,54 +769,90 @@ __global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_con
   };
 
   // One capsule of the warp into shared memory.
-  auto place = [&](int slot, long long g, float4 a, float4 b, const screen_rect& r, int start) {
+  auto place = [&](auto bands, int slot, long long g, float4 a, float4 b, const screen_rect& r, const screen_band& band, int start) {
     const float length2 = r.along.x * r.along.x + r.along.y * r.along.y;
     a.w = __uint_as_float((unsigned int)g);
     b.w = r.nearest;
-    entries[warp][slot] = entry {a, b, make_float4(r.from.x, r.from.y, r.along.x, r.along.y),
-                                 length2 > 1e-12f ? __frcp_rn(length2) : 0.0f, r.radius2, __frcp_rn(float(r.w)), r.w, r.x0, r.y0, start, 0};
+    entry& E = entries[warp][slot];
+    E.a = a; E.b = b;
+    E.line = make_float4(r.from.x, r.from.y, r.along.x, r.along.y);
+    E.inverse_length2 = length2 > 1e-12f ? __frcp_rn(length2) : 0.0f;
+    E.radius2 = r.radius2;
+    E.inverse_w = __frcp_rn(float(band.w));
+    E.w = band.w;
+    E.start = start;
+    E.pixel = r.y0 * A.width + r.x0;
+    if constexpr (decltype(bands)::value)
+    {
+      E.across = band.columns ? r.h : r.w;
+      E.columns = band.columns;
+      E.slope = band.slope;
+      E.base = band.base;
+    }
   };
 
   // The pixels [begin, end) of the warp's rectangles, laid one after the other;
   // `placed` capsules in shared memory.
-  auto walk = [&](int begin, int end, int placed) {
+  // Bands: the rows may be narrower than the rectangles, and two turns go together.
+  auto walk = [&](auto bands, int begin, int end, int placed) {
+    constexpr bool BANDS = decltype(bands)::value;
+    constexpr int turns = BANDS ? 2 : 1;
     const int own_start = lane < placed ? entries[warp][lane].start : INT_MAX;
     int before = begin > 0 ? 0 : -1;               // the capsule whose pixels the turn begins in, or just before it
     int queued = 0;
-    for (int base = begin; base < end; base += 32)
+    for (int base = begin; base < end; base += 32 * turns)
     {
-      const unsigned begins = __reduce_or_sync(0xffffffffu, own_start >= base && own_start < base + 32 ? 1u << (own_start - base) : 0u);
-      const int i = base + lane;
-      bool wanted = false;
-      uint2 item = make_uint2(0, 0);
-      if (i < end)
+      // (the keys of two turns are on the way at the same time)
+      bool wanted[turns] = {};
+      uint2 item[turns];
+      #pragma unroll
+      for (int u = 0; u < turns; ++u)
       {
-        const int c = before + __popc(begins & (lanes_below | (1u << lane)));
-        const entry& E = entries[warp][c];
-        // (rectangles of at most 2^20 pixels: the product's error stays below half a pixel's share)
-        const int local = i - E.start, row = int((float(local) + 0.5f) * E.inverse_w), column = local - row * E.w;
-        const float qx = float(column) - E.line.x, qy = float(row) - E.line.y;
-        const float t = __saturatef(__fmaf_rn(qx, E.line.z, qy * E.line.w) * E.inverse_length2);
-        const float ex = __fmaf_rn(-t, E.line.z, qx), ey = __fmaf_rn(-t, E.line.w, qy);
-        if (!(__fmaf_rn(ex, ex, ey * ey) > E.radius2))
+        const int from = base + 32 * u, i = from + lane;
+        if (u > 0 && from >= end) break;
+        const unsigned begins = __reduce_or_sync(0xffffffffu, own_start >= from && own_start < from + 32 ? 1u << (own_start - from) : 0u);
+        if (i < end)
         {
-          item = make_uint2(unsigned(c), unsigned((E.y0 + row) * A.width + E.x0 + column));
-          // (a key read late is only larger: the test is then made for nothing)
-          const unsigned int nearest = __ldcg(reinterpret_cast<const unsigned int*>(A.keys + item.y) + 1);
-          wanted = nearest == 0xffffffffu || __uint_as_float(nearest) >= E.b.w;
+          const int c = before + __popc(begins & (lanes_below | (1u << lane)));
+          const entry& E = entries[warp][c];
+          // (rectangles of at most 2^20 pixels: the product's error stays below half a pixel's share)
+          const int local = i - E.start, along = int((float(local) + 0.5f) * E.inverse_w);
+          int across = local - along * E.w;
+          if constexpr (BANDS) across += int(ceilf(__fmaf_rn(E.slope, float(along), E.base)));
+          const bool columns = BANDS && E.columns;
+          const int row = columns ? across : along, column = columns ? along : across;
+          const float qx = float(column) - E.line.x, qy = float(row) - E.line.y;
+          const float t = __saturatef(__fmaf_rn(qx, E.line.z, qy * E.line.w) * E.inverse_length2);
+          const float ex = __fmaf_rn(-t, E.line.z, qx), ey = __fmaf_rn(-t, E.line.w, qy);
+          if ((!BANDS || unsigned(across) < unsigned(E.across)) && !(__fmaf_rn(ex, ex, ey * ey) > E.radius2))
+          {
+            item[u] = make_uint2(unsigned(c), unsigned(E.pixel + row * A.width + column));
+            wanted[u] = true;
+          }
+        }
+        before += __popc(begins);
+      }
+      // (a key read late is only larger: the test is then made for nothing)
+      unsigned int nearest[turns];
+      #pragma unroll
+      for (int u = 0; u < turns; ++u)
+        nearest[u] = wanted[u] ? __ldcg(reinterpret_cast<const unsigned int*>(A.keys + item[u].y) + 1) : 0u;
+      #pragma unroll
+      for (int u = 0; u < turns; ++u)
+      {
+        if (u > 0 && base + 32 * u >= end) break;
+        if (wanted[u]) wanted[u] = nearest[u] == 0xffffffffu || __uint_as_float(nearest[u]) >= entries[warp][item[u].x].b.w;
+        const unsigned mask = __ballot_sync(0xffffffffu, wanted[u]);
+        if (wanted[u]) queue[queued + __popc(mask & lanes_below)] = item[u];
+        queued += __popc(mask);
+        __syncwarp();
+        if (queued >= 32)
+        {
+          queued -= 32;
+          test(queue[queued + lane]);
+          __syncwarp();
         }
       }
-      const unsigned mask = __ballot_sync(0xffffffffu, wanted);
-      if (wanted) queue[queued + __popc(mask & lanes_below)] = item;
-      queued += __popc(mask);
-      __syncwarp();
-      if (queued >= 32)
-      {
-        queued -= 32;
-        test(queue[queued + lane]);
-        __syncwarp();
-      }
-      before += __popc(begins);
     }
     if (lane < queued) test(queue[lane]);
     __syncwarp();                                  // before the next capsules take the shared memory
@@ -800,7 +871,14 @@ __global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_con
       b = A.vertices[g + 1];
       r = project_capsule(A, a, b, jitter);
     }
-    const int area = r.w * r.h > raster_slice ? 0 : r.w * r.h;
+    int area = r.w * r.h > raster_slice ? 0 : r.w * r.h;
+    screen_band band {0, r.w, 0.0f, 0.0f};
+    const bool bands = __any_sync(0xffffffffu, area > 16);
+    if (bands && area)
+    {
+      band = band_of(r);
+      area = band.w * (band.columns ? r.w : r.h);
+    }
     int end = area;
     for (int off = 1; off < 32; off <<= 1)
     {
@@ -809,9 +887,13 @@ __global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_con
     }
     const int total = __shfl_sync(0xffffffffu, end, 31);
     const unsigned covered = __ballot_sync(0xffffffffu, area != 0);
-    if (area) place(__popc(covered & lanes_below), g, a, b, r, end - area);
-    __syncwarp();
-    walk(0, total, __popc(covered));
+    auto draw = [&](auto with_bands) {
+      if (area) place(with_bands, __popc(covered & lanes_below), g, a, b, r, band, end - area);
+      __syncwarp();
+      walk(with_bands, 0, total, __popc(covered));
+    };
+    if (bands) draw(std::true_type {});
+    else draw(std::false_type {});
   }
   const int slices = int(A.count[3]);
   for (long long s = (long long)blockIdx.x * (raster_threads / 32) + warp; s < slices; s += warps)
@@ -820,10 +902,10 @@ __global__ void __launch_bounds__(raster_threads) raster_kernel(const __grid_con
     const long long g = A.prim_vertex[slice.x];
     const float4 a = A.vertices[g], b = A.vertices[g + 1];
     const screen_rect r = project_capsule(A, a, b, jitter);
-    if (lane == 0) place(0, g, a, b, r, 0);
+    if (lane == 0) place(std::true_type {}, 0, g, a, b, r, screen_band {0, r.w, 0.0f, 0.0f}, 0);
     __syncwarp();
     const int begin = int(slice.y) * raster_slice;
-    walk(begin, min(begin + raster_slice, r.w * r.h), 1);
+    walk(std::true_type {}, begin, min(begin + raster_slice, r.w * r.h), 1);
   }
 }
 

@@ -90,3 +90,25 @@ def test_every_srgb_code_is_the_thresholds_code(ctx, port):
         assert np.array_equal(got, expected)
         seen |= set(got[..., :3].ravel().tolist())
     assert len(seen) > 150
+
+
+@pytest.mark.parametrize("radius", [0.001, 0.01, 0.05])
+def test_thin_segments_at_every_angle_equal_the_oracle(ctx, port, radius):
+    """Bands along rows and columns: slopes through 0, 1 and infinity, both directions,
+    some ending beyond the image."""
+    angle = np.linspace(0, 2 * np.pi, 49)
+    v = np.zeros((98, 4), np.float32)
+    for k, (at, length) in enumerate(zip(angle, np.resize([0.3, 1.0, 3.0], 49))):
+        centre = np.array([0.3 * np.cos(7 * at), 0.3 * np.sin(5 * at), 0.2 * np.sin(at)])
+        along = np.array([np.cos(at), np.sin(at), 0.1 * np.cos(3 * at)]) * length
+        v[2 * k, :3], v[2 * k + 1, :3] = centre, centre + along
+    c = np.random.default_rng(3).uniform(0, 1, (98, 4)).astype(np.float32)
+    batches = [(v, c, np.arange(0, 97, 2, dtype=np.int32))]
+    view = ((0.0, 0.0, -3.0), (0.0, 0.0, 1.0), (0.0, 1.0, 0.0))
+    ctx.ray_tracer_clear_volume()
+    ctx.ray_tracer_set_integral_curves_host(batches, radius)
+    ctx.ray_tracer_set_image_size(301, 233)
+    ctx.ray_tracer_set_camera(*view)
+    ctx.ray_tracer_trace(2)
+    expected, _ = port.render(batches, radius, view, (301, 233), frames=2)
+    assert np.array_equal(ctx.ray_tracer_serialize(), expected)
