@@ -347,11 +347,18 @@ struct variant
 
 // Launch shapes the autotuner chooses from, per job class: threads per CTA and
 // the minimum resident CTAs per SM that the register allocation must allow.
+// Unsteady jobs wait for two slices' corners: 16 warps per SM (128 registers)
+// instead of the 12 that 150 registers leave take 1160 instead of 2190 us for six
+// fields of 32^3 to 128^3 and 400 steps, 1362 instead of 1838 for 120000 seeds on
+// 100^3 and 300 steps, 4020 instead of 4615 for 500000 on 128^3 and 200 steps (20
+// warps, 96 registers and spills: 1470 for the first).  Seeds that leave 12 warps
+// idle anyway take the 150 registers (batch_shape): 30000 seeds 693 us, 757 with
+// 128; 4000 seeds 286, 310.
 const variant variants[batch_classes][4] = {
   {PARS_BATCH_VARIANT(64, 1, batch_steady), PARS_BATCH_VARIANT(128, 1, batch_steady),
    PARS_BATCH_VARIANT(128, 5, batch_steady), PARS_BATCH_VARIANT(256, 1, batch_steady)},
-  {PARS_BATCH_VARIANT(64, 1, batch_unsteady), PARS_BATCH_VARIANT(128, 1, batch_unsteady),
-   PARS_BATCH_VARIANT(128, 3, batch_unsteady), PARS_BATCH_VARIANT(256, 1, batch_unsteady)},
+  {PARS_BATCH_VARIANT(64, 8, batch_unsteady), PARS_BATCH_VARIANT(128, 4, batch_unsteady),
+   PARS_BATCH_VARIANT(128, 3, batch_unsteady), PARS_BATCH_VARIANT(256, 2, batch_unsteady)},
   {PARS_BATCH_VARIANT(64, 1, batch_frozen), PARS_BATCH_VARIANT(128, 1, batch_frozen),
    PARS_BATCH_VARIANT(128, 6, batch_frozen), PARS_BATCH_VARIANT(256, 1, batch_frozen)},
 };
@@ -367,7 +374,14 @@ int batch_resident_warps(pars_gpu_context& ctx, int job_class, int v)
   if (per_sm < 0) PARS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, var.kernel, var.threads, 0));
   return per_sm * var.threads / 32;
 }
-int batch_variant_threads(int v) { return variants[0][v].threads; }
+int batch_variant_threads(int job_class, int v) { return variants[job_class][v].threads; }
+int batch_shape(pars_gpu_context& ctx, int job_class, long long seeds)
+{
+  if (job_class != batch_unsteady) return ctx.batch_variant[job_class];
+  if (ctx.sm_count <= 0) PARS_CUDA(cudaDeviceGetAttribute(&ctx.sm_count, cudaDevAttrMultiProcessorCount, ctx.device));
+  return seeds <= 32LL * batch_resident_warps(ctx, job_class, batch_unsteady_few) * ctx.sm_count ? batch_unsteady_few
+                                                                                                  : ctx.batch_variant[job_class];
+}
 int batch_pool_seeds() { return pool_seeds; }
 
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int v, const batch_job_device* jobs, int njobs,

@@ -466,7 +466,10 @@ enum batch_class { batch_steady = 0, batch_unsteady = 1, batch_frozen = 2, batch
 int  batch_variant_count();
 // Resident warps per SM of a job class's launch shape.
 int  batch_resident_warps(pars_gpu_context& ctx, int job_class, int variant);
-int  batch_variant_threads(int variant);
+int  batch_variant_threads(int job_class, int variant);
+// The launch shape of an untold launch: the tuned one, but for few unsteady seeds.
+int  batch_shape(pars_gpu_context& ctx, int job_class, long long seeds);
+constexpr int batch_unsteady_few = 2;   // not a candidate of the tuning
 int  batch_pool_seeds();
 // job_class: batch_steady, batch_unsteady or batch_frozen.
 void launch_batch_advect(pars_gpu_context& ctx, int job_class, int variant, const batch_job_device* jobs, int njobs,

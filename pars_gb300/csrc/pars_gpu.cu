@@ -913,6 +913,7 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
   // resident warps per SM (on the 256^3 flow map the 96-register shape, five
   // CTAs of 128, beats the 104-register ones by 7 %, which the probes alone
   // do not resolve reliably).
+  if (c == batch_unsteady) fastest[batch_unsteady_few] = INFINITY;   // chosen by the seeds (batch_shape)
   const float best_time = *std::min_element(fastest.begin(), fastest.end());
   int best_v = -1, best_warps = -1;
   for (int v = 0; v < batch_variant_count(); ++v)
@@ -981,7 +982,7 @@ std::vector<unsigned long long> execute_batch(pars_gpu_context& ctx, std::vector
   PARS_CUDA(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * (count + C), ctx.stream));
   for (int c = 0; c < C; ++c)
     if (size[c] > 0)
-      launch_batch_advect(ctx, c, variant >= 0 ? variant : ctx.batch_variant[c], device_jobs + first[c], size[c], pools[c], seeds[c],
+      launch_batch_advect(ctx, c, variant >= 0 ? variant : batch_shape(ctx, c, seeds[c]), device_jobs + first[c], size[c], pools[c], seeds[c],
                           counters + c);
   std::vector<unsigned long long> steps(count + C);
   PARS_CUDA(cudaMemcpyAsync(steps.data(), counters, sizeof(unsigned long long) * (count + C), cudaMemcpyDeviceToHost, ctx.stream));
@@ -1114,7 +1115,7 @@ long long engine_submit(pars_gpu_context& ctx, const batch_job_device& job)
   batch_job_device j = job;
   j.clock = make_slice_clock(j.time, j.time_begin, j.rule.h);
   if (ctx.batch_variant[c] < 0) tune_class(ctx, c, {j});
-  if (E.open == 0) E.variant = ctx.batch_variant[c];   // fixed while the class has work
+  if (E.open == 0) E.variant = batch_shape(ctx, c, j.seed_count);   // fixed while the class has work
   engine_reserve(ctx, E, int(E.jobs.size()) + 1);
   j.first_pool = E.total_pools;
   j.steps = E.counters.as<unsigned long long>() + 4 + E.jobs.size();
@@ -2023,7 +2024,7 @@ int32_t pars_gpu_batch_tuned(pars_gpu_context* ctx, int32_t job_class, int32_t* 
     PARS_REQUIRE(job_class >= 0 && job_class < batch_classes, "job_class is 0 (steady), 1 (unsteady) or 2 (frozen)");
     const int v = ctx->batch_variant[job_class];
     if (variant) *variant = v;
-    if (threads) *threads = v >= 0 ? batch_variant_threads(v) : 0;
+    if (threads) *threads = v >= 0 ? batch_variant_threads(job_class, v) : 0;
   });
 }
 
