@@ -78,12 +78,11 @@ __device__ __forceinline__ void flow_step(const flow_map_args& a, corner_cache& 
 // whole call).
 // Frozen steps need few registers once the corners are cached: seven CTAs of 128
 // per SM (72 registers) took 4.0 ms where 80 registers took 4.3 and 94 took 4.4
-// (150 x 128 x 141 vertices, 300 steps).  RK4 / Euler and Adams: five (96
-// registers); the tableaux keep what the compiler chooses (95 to 112).
-constexpr int flow_min_ctas(int scheme)
-{
-  return scheme == flow_frozen ? 7 : scheme == flow_classic || scheme >= flow_adams_bashforth ? 5 : 1;
-}
+// (150 x 128 x 141 vertices, 300 steps).  The others: five (96 registers); the
+// tableaux, which took what the compiler chose before (95 to 112), 3489 -> 3386 us
+// (Dormand-Prince, 100^3, 200 steps) and 7858 -> 7375 us (Fehlberg 7(8)), 64^3
+// within 3 %.
+constexpr int flow_min_ctas(int scheme) { return scheme == flow_frozen ? 7 : 5; }
 
 template <int SCHEME>
 __global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(const __grid_constant__ flow_map_args a, refill_rule refill)
