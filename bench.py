@@ -4,7 +4,7 @@
 Workload (one "step"): the FTLE pipeline on a 256^3 FP32 ABC flow plus
 N(0, 0.01) noise (seed 0): one seed per grid vertex (16,777,216 particles),
 classical RK4 with four field samples per step, h = 0.01, at most 500 steps
-(T = 5), flow map, then the fused gradient / Cauchy-Green / Jacobi eigenvalue /
+(T = 5), flow map, then the fused gradient / Cauchy-Green / largest eigenvalue /
 log FTLE kernel (FP32).  Metric: RK4 particle-steps per second (steps actually
 taken), with FTLE voxels per second beside it.
 
@@ -34,7 +34,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "RK4 particle-steps/s"
 UNIT = "particle-steps/s"
-BYTES_PER_RK4_STEP = 512          # 4 samples x 8 corners x 16 B (flow-map mode: no vertex store)
+BYTES_PER_RK4_STEP = 384          # 4 samples x (4 corners x 16 B + 4 x 8 B) (flow-map mode: no vertex store)
 BYTES_PER_FTLE_VOXEL = 100        # 6 neighbour float4 reads + one FP32 write
 
 
@@ -855,7 +855,7 @@ def main():
     max_steps = args.iterations - 1
     config = {"workload": f"ftle_{n}: ABC + N(0,0.01) noise (seed 0) on {n}^3 FP32 vertices of [0,2pi]^3, one seed per vertex "
                           f"({seeds} particles), classical RK4 (4 samples/step) h=0.01, <= {max_steps} steps (T=5), "
-                          "flow map + fused central-difference / Cauchy-Green / FP32 Jacobi eigenvalue / log FTLE",
+                          "flow map + fused central-difference / Cauchy-Green / largest eigenvalue / log FTLE",
               "grid": n, "seeds": seeds, "max_steps": max_steps, "step_size": 0.01, "stage_mode": "resampled",
               "field_samples_per_step": 4, "reference_field_samples_per_step": 1,
               "ranks": world, "l2": f"inputs larger than L2 ({16 * n ** 3 / 1e6:.0f} MB float4 field) and a 256 MB L2 flush "

@@ -294,7 +294,7 @@ int32_t pars_gpu_flow_map_generate(pars_gpu_context* context, int32_t field, int
                                    int32_t integrator, int32_t stage_mode, float step_size, int32_t* flow_map, int64_t* steps);
 /* FTLE of a flow-map field: central-difference gradient (one-sided at the
  * borders), Cauchy-Green tensor C (FP32), then log(sqrt(lambda_max)) / |time|
- * with lambda_max from cyclic Jacobi rotations (mode REGULAR), or the
+ * with lambda_max from Eberly's construction in FP32 (mode REGULAR), or the
  * fractional anisotropy of C's eigenvalues (mode FRACTIONAL_ANISOTROPY,
  * ftle_map_generator.cpp:51-54).  Writes
  * the FP32 field to HOST `ftle` (X*Y*Z floats) unless it is NULL, in which case
