@@ -219,9 +219,8 @@ cudaError_t launch_flow_map_kernel(const flow_map_args& a, flow_scheme scheme, i
 // each (random, near-degenerate, near-isotropic, strongly anisotropic): rms 3.2e-8
 // to 4.6e-8, largest 1.6e-7; the cyclic Jacobi sweeps that this replaces (12
 // rotations with two divisions and a square root each): 3.4e-8 to 6.2e-8, largest
-// 2.7e-7.  The FTLE of 320 x 300 x 311 vertices: 1.47 -> 0.49 ms, with
-// coordinate_difference and quotient below; still bound by FP32 and integer
-// issue (its 597 MB take 0.09 ms).
+// 2.7e-7.  The FTLE of 320 x 300 x 311 vertices: 1.47 -> 0.46 ms, with the decoding
+// and the quotients below (its 597 MB take 0.09 ms).
 __device__ __forceinline__ float largest_eigenvalue(float c00, float c11, float c22, float c01, float c02, float c12)
 {
   const float trace = c00 + c11 + c22;
@@ -239,8 +238,11 @@ __device__ __forceinline__ float largest_eigenvalue(float c00, float c11, float 
   const float q = (c00 + c11 + c22) * (1.0f / 3.0f);
   const float d0 = c00 - q, d1 = c11 - q, d2 = c22 - q;
   const float off = fmaf(c01, c01, fmaf(c02, c02, c12 * c12));
-  const float p = __fsqrt_rn(fmaf(2.0f, off, fmaf(d0, d0, fmaf(d1, d1, d2 * d2))) * (1.0f / 6.0f));
-  const float inv = p > 1e-18f ? __frcp_rn(p) : 0.0f;
+  const float p2 = fmaf(2.0f, off, fmaf(d0, d0, fmaf(d1, d1, d2 * d2))) * (1.0f / 6.0f);
+  // p and 1 / p from one reciprocal root, each with a Newton step
+  const float y = p2 > 1e-36f ? rsqrtf(p2) : 0.0f, p0 = p2 * y;
+  const float p = fmaf(0.5f * y, fmaf(-p0, p0, p2), p0);
+  const float inv = fmaf(y, fmaf(-p, y, 1.0f), y);
   const float b00 = d0 * inv, b11 = d1 * inv, b22 = d2 * inv, b01 = c01 * inv, b02 = c02 * inv, b12 = c12 * inv;
   const float m0 = fmaf(b11, b22, -b12 * b12), m1 = fmaf(b01, b22, -b12 * b02), m2 = fmaf(b01, b12, -b11 * b02);
   const float det = fmaf(b00, m0, fmaf(-b01, m1, b02 * m2));
@@ -292,59 +294,81 @@ struct ftle_args
   float         width[3], inverse_width[3];   // 2 h per axis and its reciprocal
   float         inverse_time;     // 1 / |T|
   int           mode;
+  int           planes;           // 1: a row of CTAs per x plane; 0: one row over all vertices
   float*        out;
 };
 
 // x / d; y = RN(1 / d), 0 for a width whose reciprocal leaves the normal range.
 __device__ __forceinline__ float quotient(float x, float d, float y) { return y == 0.0f ? __fdiv_rn(x, d) : quotient_rn(x, d, y); }
 
-// b - a of two coordinates with residual codes in bits [shift, shift + 10) of
-// wb, wa (residual_value): the difference of the residuals, code 2^e(b) -
-// code 2^e(a) up to the common factor 2^-23 / 1022, is one FMA and exact for
-// neighbours of the same binade.
-__device__ __forceinline__ float residual_code(unsigned w, int shift)
+// A flow-map position: its stored coordinates and its residuals (code 2^e; the
+// factor 2^-23 / 1022 is left out, so they are exact).
+struct flow_vertex
 {
-  // the 10-bit code plus 512 as the low mantissa bits of 2^23
-  return __uint_as_float(((w >> shift) & 0x3ffu) ^ 0x4b000200u) - 8389120.0f;
-}
+  float3 x, r;
+};
 __device__ __forceinline__ float binade(float x) { return __uint_as_float(__float_as_uint(x) & 0x7f800000u); }
-__device__ __forceinline__ float coordinate_difference(float b, unsigned wb, float a, unsigned wa, int shift)
+__device__ __forceinline__ flow_vertex load_vertex(const ftle_args& a, const float4* p)
 {
-  const float r = fmaf(residual_code(wb, shift), binade(b), -residual_code(wa, shift) * binade(a));
-  return fmaf(r, 0x1p-23f / 1022.0f, __fsub_rn(b, a));
+  const float4 v = __ldg(p);
+  const unsigned w = __float_as_uint(v.w) & a.codes;
+  // each 10-bit code plus 512 as mantissa bits of a power of two: bits 0-9 of
+  // 2^23, bits 10-19 of 2^13, bits 20-29 (shifted down) of 2^23
+  return {make_float3(v.x, v.y, v.z), make_float3((__uint_as_float((w & 0x3ffu) ^ 0x4b000200u) - 8389120.0f) * binade(v.x),
+                                                  (__uint_as_float((w & 0xffc00u) ^ 0x46080000u) - 8704.0f) * binade(v.y),
+                                                  (__uint_as_float(((w >> 20) & 0x3ffu) ^ 0x4b000200u) - 8389120.0f) * binade(v.z))};
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) ftle_kernel(const ftle_args a)
+// b - a: the FP32 difference of neighbouring coordinates is exact where they lie
+// within a factor of two of each other (Sterbenz); the residuals' difference, exact
+// for neighbours of the same binade, is added to it.
+__device__ __forceinline__ float difference(float b, float rb, float a, float ra)
 {
-  const long long total = (long long)a.nx * a.ny * a.nz;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  int idx[3];
-  lattice_index(i, a.ny, a.nz, idx[0], idx[1], idx[2]);
+  return fmaf(__fsub_rn(rb, ra), 0x1p-23f / 1022.0f, __fsub_rn(b, a));
+}
 
-  // Column j of J: (phi(+e_j) - phi(-e_j)) / (2 h_j), one-sided at borders.
-  float J[3][3];
-  const int   ext[3] = {a.nx, a.ny, a.nz};
-  const long long stride[3] = {(long long)a.ny * a.nz, a.nz, 1};
-  #pragma unroll
-  for (int j = 0; j < 3; ++j)
+// Column j of J: (phi(+e_j) - phi(-e_j)) / (2 h_j); a one-sided difference divides
+// by h_j (half the width, exactly).
+__device__ __forceinline__ float3 jacobian_column(const ftle_args& a, int j, const flow_vertex& hi, const flow_vertex& lo, bool one_sided)
+{
+  const float width = one_sided ? 0.5f * a.width[j] : a.width[j], inverse = one_sided ? 2.0f * a.inverse_width[j] : a.inverse_width[j];
+  return make_float3(quotient(difference(hi.x.x, hi.r.x, lo.x.x, lo.r.x), width, inverse),
+                     quotient(difference(hi.x.y, hi.r.y, lo.x.y, lo.r.y), width, inverse),
+                     quotient(difference(hi.x.z, hi.r.z, lo.x.z, lo.r.z), width, inverse));
+}
+
+// One vertex per thread.  Bound by instruction issue (88 % of the cycles), so the
+// place in the lattice costs one 32-bit division (CTAs by x plane), the codes are
+// decoded by masks, and a column's borders by selects: 320 x 300 x 311 vertices 491
+// -> 460 us with the reciprocal root above, 256^3 278 -> 261, 150 x 128 x 141 51 ->
+// 49.  (16 planes per thread, the vertices at x - 1 and x kept decoded: 446, 253, 49,
+// but 64^3 12 instead of 11: not worth a second kernel.)
+template <int MODE>
+__global__ void __launch_bounds__(256) ftle_kernel(const __grid_constant__ ftle_args a)
+{
+  const long long plane = (long long)a.ny * a.nz, p = (long long)blockIdx.x * 256 + threadIdx.x;
+  int x, y, z;
+  if (a.planes)
   {
-    if (ext[j] == 1) { J[0][j] = J[1][j] = J[2][j] = 0.0f; continue; }
-    const bool first = idx[j] == 0, last = idx[j] == ext[j] - 1;
-    const long long lo = first ? i : i - stride[j], hi = last ? i : i + stride[j];
-    // positions with their sub-ulp residuals (code 0: none); the FP32
-    // difference of neighbouring coordinates is exact where they lie within a
-    // factor of two of each other (Sterbenz), the residuals' difference is
-    // added to it
-    const float4 A = __ldg(a.flow + lo), B = __ldg(a.flow + hi);
-    const unsigned wa = __float_as_uint(A.w) & a.codes, wb = __float_as_uint(B.w) & a.codes;
-    // a one-sided difference is doubled (exactly), so every axis divides by 2 h
-    const float twice = first || last ? 2.0f : 1.0f;
-    J[0][j] = quotient(twice * coordinate_difference(B.x, wb, A.x, wa, 0), a.width[j], a.inverse_width[j]);
-    J[1][j] = quotient(twice * coordinate_difference(B.y, wb, A.y, wa, 10), a.width[j], a.inverse_width[j]);
-    J[2][j] = quotient(twice * coordinate_difference(B.z, wb, A.z, wa, 20), a.width[j], a.inverse_width[j]);
+    if (p >= plane) return;
+    x = int(blockIdx.y);
+    y = int(unsigned(p) / unsigned(a.nz));
+    z = int(p) - y * a.nz;
   }
+  else
+  {
+    if (p >= plane * a.nx) return;
+    lattice_index(p, a.ny, a.nz, x, y, z);
+  }
+  const long long i = ((long long)x * a.ny + y) * a.nz + z;
+  const float4* v = a.flow + i;
+  const float4 *x_lo = x == 0 ? v : v - plane, *x_hi = x == a.nx - 1 ? v : v + plane;
+  const int y_lo = y == 0 ? 0 : a.nz, y_hi = y == a.ny - 1 ? 0 : a.nz, z_lo = z == 0 ? 0 : 1, z_hi = z == a.nz - 1 ? 0 : 1;
+  const float3 none = make_float3(0.f, 0.f, 0.f);   // the column of an axis of one vertex
+  const float3 J0 = a.nx > 1 ? jacobian_column(a, 0, load_vertex(a, x_hi), load_vertex(a, x_lo), x_lo == v || x_hi == v) : none;
+  const float3 J1 = a.ny > 1 ? jacobian_column(a, 1, load_vertex(a, v + y_hi), load_vertex(a, v - y_lo), y_lo == 0 || y_hi == 0) : none;
+  const float3 J2 = a.nz > 1 ? jacobian_column(a, 2, load_vertex(a, v + z_hi), load_vertex(a, v - z_lo), z_lo == 0 || z_hi == 0) : none;
+  const float J[3][3] = {{J0.x, J1.x, J2.x}, {J0.y, J1.y, J2.y}, {J0.z, J1.z, J2.z}};
   // Cauchy-Green tensor C = J^T J (FP32) and its eigenvalues.
   float C[3][3];
   #pragma unroll
@@ -383,8 +407,12 @@ void set_widths(ftle_args& a, float hx, float hy, float hz)
   for (int j = 0; j < 3; ++j) { a.width[j] = 2.0f * h[j]; a.inverse_width[j] = h[j] > 1e-30f && h[j] < 1e30f ? 1.0f / a.width[j] : 0.0f; }
 }
 
-void launch_ftle_kernel(const ftle_args& a, unsigned grid, cudaStream_t stream)
+void launch_ftle_kernel(ftle_args& a, cudaStream_t stream)
 {
+  // by plane where its last CTA is a small part of it
+  const long long plane = (long long)a.ny * a.nz;
+  a.planes = plane >= 4096 && plane < (1LL << 31) && a.nx <= 65535 ? 1 : 0;
+  const dim3 grid((unsigned)(((a.planes ? plane : plane * a.nx) + 255) / 256), a.planes ? (unsigned)a.nx : 1u);
   if (a.mode == PARS_FTLE_REGULAR) ftle_kernel<PARS_FTLE_REGULAR><<<grid, 256, 0, stream>>>(a);
   else                             ftle_kernel<PARS_FTLE_FRACTIONAL_ANISOTROPY><<<grid, 256, 0, stream>>>(a);
 }
@@ -425,7 +453,7 @@ void launch_ftle(pars_gpu_context& ctx, const field_view& flow, double time, int
   const long long total = (long long)a.nx * a.ny * a.nz;
   if (total <= 0) return;
   launch_scope scope(ctx, "ftle_fused");
-  launch_ftle_kernel(a, (unsigned)((total + 255) / 256), ctx.stream);
+  launch_ftle_kernel(a, ctx.stream);
 }
 
 // ---- Allocation-free FTLE ------------------------------------------------------
@@ -578,7 +606,7 @@ extern "C" int32_t pars_gpu_ftle_no_alloc(const float* device_xyz, const int32_t
   t.inverse_time = float(1.0 / fabs(double(time)));
   t.mode = mode;
   t.out = device_ftle;
-  launch_ftle_kernel(t, (unsigned)((voxels + 255) / 256), s);
+  launch_ftle_kernel(t, s);
   if (cudaGetLastError() != cudaSuccess) return PARS_ERR_CUDA;
   if (device_steps) steps_to_int64_kernel<<<1, 1, 0, s>>>(counter, device_steps);
   if (cudaGetLastError() != cudaSuccess) return PARS_ERR_CUDA;

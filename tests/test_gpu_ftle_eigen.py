@@ -64,3 +64,15 @@ def test_planar_and_degenerate_maps(ctx):
             i[a] += s
             touched[tuple(i)] = True
     assert np.all(np.isnan(got[touched])) and np.all(np.isfinite(got[~touched]))
+
+
+@pytest.mark.parametrize("shape", [(2, 64, 64), (3, 63, 65), (3, 64, 65), (5, 2, 2048), (4, 2, 2049), (66000, 2, 2)])
+def test_planes_and_ragged_lattices_against_fp64(ctx, shape):
+    """Either side of the change from CTAs by plane to one row over all vertices."""
+    rng = np.random.default_rng(sum(shape))
+    h = 0.25
+    grid = np.stack(np.meshgrid(*[np.arange(n) * h for n in shape], indexing="ij"), -1)
+    p = (grid + 0.1 * rng.normal(size=grid.shape)).astype(np.float32)
+    got, expected = _run(ctx, p, h), _ftle64(p, h)
+    # relative to lambda: the logarithm's absolute error, and two ulps of its value
+    assert np.all(np.abs(got - expected) <= TOLERANCE + 2.0 ** -22 * np.abs(expected))
