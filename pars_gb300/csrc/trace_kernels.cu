@@ -163,11 +163,14 @@ __device__ __forceinline__ void add_steps(const trace_launch& a, unsigned int st
 // One particle per thread, `lanes` of a warp's threads used: for launches with no
 // more particles than resident lanes, where refilling cannot help and warp votes
 // would only add latency.
+// These launches have at most 16 warps per SM, which leaves a thread 128 registers;
+// the compiler's own choice for CTAs of 32 was 96: 483 -> 455 us (4096 particles of
+// 1000 steps, 64^3), 332 -> 309 (512), 666 -> 634 (12167 of 800, 141^3).
 // FETCH (re-sampled RK4 on fields that do not stay in L2): a step's stages lie in
 // other cells, and each waits for its corners before the next is known; the end
 // cell's are fetched while the middle ones are sampled.
 template <int MODE, bool FETCH = false>
-__global__ void __launch_bounds__(32) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
+__global__ void __launch_bounds__(32, 16) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
 {
   unsigned int slot = 0;
   if constexpr (FETCH)
