@@ -582,7 +582,11 @@ struct screen_rect
 };
 
 // Rectangles above raster_slice pixels are cut into slices of that many, which any
-// warp may take; the others are walked by the warp that projects them.
+// warp may take; the others are walked by the warp that projects them.  The slices
+// are listed once for all frames of a call, while a frame's jitter moves a
+// rectangle's edges by up to a pixel, so which rectangles are large, and their
+// pixels, must not depend on the frame: a capsule that some jitter makes large is
+// drawn through the rectangle of all jitters in every frame.
 constexpr int raster_slice = 2048, raster_slices = 1 << 16;
 
 __device__ __forceinline__ float largest3(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
@@ -614,11 +618,19 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   const float left = x_lo * (x_lo < 0.0f ? i0 : i1), right = x_hi * (x_hi > 0.0f ? i0 : i1);
   const float top = -y_hi * (y_hi > 0.0f ? i0 : i1), bottom = -y_lo * (y_lo < 0.0f ? i0 : i1);
   auto margin = [](float v) { return 0.0625f + fabsf(v) * 1e-6f; };
-  const float fx0 = ceilf(cx + left - margin(left)), fx1 = floorf(cx + right + margin(right));
-  const float fy0 = ceilf(cy + top - margin(top)), fy1 = floorf(cy + bottom + margin(bottom));
-  const int x0 = int(fminf(fmaxf(fx0, 0.0f), float(A.width))), x1 = int(fmaxf(fminf(fx1, float(A.width - 1)), -1.0f));
-  const int y0 = int(fminf(fmaxf(fy0, 0.0f), float(A.height))), y1 = int(fmaxf(fminf(fy1, float(A.height - 1)), -1.0f));
+  auto first = [&](float c, float v, int size) { return int(fminf(fmaxf(ceilf(c + v - margin(v)), 0.0f), float(size))); };
+  auto last = [&](float c, float v, int size) { return int(fmaxf(fminf(floorf(c + v + margin(v)), float(size - 1)), -1.0f)); };
+  // the rectangle of every jitter in [0, 1] (each operation is monotone, so it holds this one's)
+  const float mx = 0.5f * float(A.width), my = 0.5f * float(A.height);
+  int x0 = first(mx - 1.0f, left, A.width), x1 = last(mx, right, A.width);
+  int y0 = first(my - 1.0f, top, A.height), y1 = last(my, bottom, A.height);
   if (x1 < x0 || y1 < y0) return r;
+  if ((x1 - x0 + 1) * (y1 - y0 + 1) <= raster_slice)
+  {
+    x0 = first(cx, left, A.width); x1 = last(cx, right, A.width);
+    y0 = first(cy, top, A.height); y1 = last(cy, bottom, A.height);
+    if (x1 < x0 || y1 < y0) return r;
+  }
   r.x0 = x0; r.y0 = y0; r.w = x1 - x0 + 1; r.h = y1 - y0 + 1;
   // a point within `pad` of the segment projects within
   // pad focal sqrt(1 + slope^2) / z0 of the projected segment (sqrt(1 + s) <= 1 + s / 2)
