@@ -579,14 +579,14 @@ struct screen_rect
   float  nearest;         // a lower bound of t for hits of this capsule
   float2 from, along;     // the projected segment (pixels from the rectangle's corner) ...
   float  radius2;         // ... and the square of the distance that its hits keep to it
+  bool   large;           // drawn in slices; the same in every frame of a call, as the rectangle then is
 };
 
-// Rectangles above raster_slice pixels are cut into slices of that many, which any
-// warp may take; the others are walked by the warp that projects them.  The slices
-// are listed once for all frames of a call, while a frame's jitter moves a
-// rectangle's edges by up to a pixel, so which rectangles are large, and their
-// pixels, must not depend on the frame: a capsule that some jitter makes large is
-// drawn through the rectangle of all jitters in every frame.
+// Large rectangles are cut into slices of raster_slice pixels, which any warp may
+// take; the others are walked by the warp that projects them.  The slices are listed
+// once for all frames of a call, while a frame's jitter moves a rectangle's edges by
+// up to a pixel.  So a capsule is large or not by its extent before the jitter, and a
+// large one is drawn through the rectangle of all jitters in every frame.
 constexpr int raster_slice = 2048, raster_slices = 1 << 16;
 
 __device__ __forceinline__ float largest3(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
@@ -607,9 +607,9 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   const float pad = A.radius + (A.radius + magnitude) * (1.0f / 65536.0f);
   const float za = dot3(a, A.forward), zb = dot3(b, A.forward);
   const float z0 = fminf(za, zb) - pad, z1 = fmaxf(za, zb) + pad;
-  screen_rect r {0, 0, 0, 0, z0, {0.0f, 0.0f}, {0.0f, 0.0f}, INFINITY};
+  screen_rect r {0, 0, 0, 0, z0, {0.0f, 0.0f}, {0.0f, 0.0f}, INFINITY, false};
   if (!(z1 > 0.0f)) return r;                                   // behind the camera
-  if (!(z0 > 0.0f)) { r.w = A.width; r.h = A.height; return r; }   // around it
+  if (!(z0 > 0.0f)) { r.w = A.width; r.h = A.height; r.large = true; return r; }   // around it
   const float xa = dot3(a, A.right), xb = dot3(b, A.right), ya = dot3(a, A.up), yb = dot3(b, A.up);
   const float i0 = __fdividef(A.focal, z0), i1 = __fdividef(A.focal, z1);   // (a few ulps: far inside the margins)
   const float x_lo = fminf(xa, xb) - pad, x_hi = fmaxf(xa, xb) + pad, y_lo = fminf(ya, yb) - pad, y_hi = fmaxf(ya, yb) + pad;
@@ -620,17 +620,16 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   auto margin = [](float v) { return 0.0625f + fabsf(v) * 1e-6f; };
   auto first = [&](float c, float v, int size) { return int(fminf(fmaxf(ceilf(c + v - margin(v)), 0.0f), float(size))); };
   auto last = [&](float c, float v, int size) { return int(fmaxf(fminf(floorf(c + v + margin(v)), float(size - 1)), -1.0f)); };
-  // the rectangle of every jitter in [0, 1] (each operation is monotone, so it holds this one's)
-  const float mx = 0.5f * float(A.width), my = 0.5f * float(A.height);
-  int x0 = first(mx - 1.0f, left, A.width), x1 = last(mx, right, A.width);
-  int y0 = first(my - 1.0f, top, A.height), y1 = last(my, bottom, A.height);
-  if (x1 < x0 || y1 < y0) return r;
-  if ((x1 - x0 + 1) * (y1 - y0 + 1) <= raster_slice)
+  int x0 = first(cx, left, A.width), x1 = last(cx, right, A.width), y0 = first(cy, top, A.height), y1 = last(cy, bottom, A.height);
+  r.large = !((right - left) * (bottom - top) <= float(raster_slice));
+  if (r.large)
   {
-    x0 = first(cx, left, A.width); x1 = last(cx, right, A.width);
-    y0 = first(cy, top, A.height); y1 = last(cy, bottom, A.height);
-    if (x1 < x0 || y1 < y0) return r;
+    // of every jitter in [0, 1] (each operation is monotone, so it holds this one's)
+    const float mx = 0.5f * float(A.width), my = 0.5f * float(A.height);
+    x0 = first(mx - 1.0f, left, A.width); x1 = last(mx, right, A.width);
+    y0 = first(my - 1.0f, top, A.height); y1 = last(my, bottom, A.height);
   }
+  if (x1 < x0 || y1 < y0) return r;
   r.x0 = x0; r.y0 = y0; r.w = x1 - x0 + 1; r.h = y1 - y0 + 1;
   // a point within `pad` of the segment projects within
   // pad focal sqrt(1 + slope^2) / z0 of the projected segment (sqrt(1 + s) <= 1 + s / 2)
@@ -669,7 +668,7 @@ __device__ __forceinline__ screen_band band_of(const screen_rect& r)
 constexpr int raster_threads = 256;
 
 // The rectangles' pixels, all together and of the largest one.
-__global__ void __launch_bounds__(raster_threads) raster_count_kernel(const __grid_constant__ raster_args A)
+__global__ void __launch_bounds__(raster_threads, 8) raster_count_kernel(const __grid_constant__ raster_args A)
 {
   unsigned long long sum = 0, most = 0;
   float scene = 0.0f;
@@ -683,7 +682,7 @@ __global__ void __launch_bounds__(raster_threads) raster_count_kernel(const __gr
     const unsigned long long area = (unsigned long long)r.w * r.h;
     sum += area;
     most = max(most, area);
-    if (area > raster_slice && area <= A.limit_each)
+    if (r.large && area && area <= A.limit_each)
     {
       const unsigned long long n = (area + raster_slice - 1) / raster_slice, at = atomicAdd(A.count + 3, n);
       for (unsigned long long i = 0; i < n && at + i < raster_slices; ++i) A.slices[at + i] = make_uint2((unsigned int)k, (unsigned int)i);
@@ -873,7 +872,7 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
   for (long long first = ((long long)blockIdx.x * (raster_threads / 32) + warp) * 32; first < A.prims; first += warps * 32)
   {
     const long long k = first + lane;
-    screen_rect r {0, 0, 0, 0, 0.0f, {0.0f, 0.0f}, {0.0f, 0.0f}, 0.0f};
+    screen_rect r {0, 0, 0, 0, 0.0f, {0.0f, 0.0f}, {0.0f, 0.0f}, 0.0f, false};
     float4 a, b;
     long long g = 0;
     if (k < A.prims)
@@ -883,7 +882,7 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
       b = A.vertices[g + 1];
       r = project_capsule(A, a, b, jitter);
     }
-    int area = r.w * r.h > raster_slice ? 0 : r.w * r.h;
+    int area = r.large ? 0 : r.w * r.h;
     screen_band band {0, r.w, 0.0f, 0.0f};
     const bool bands = __any_sync(0xffffffffu, area > 16);
     if (bands && area)
