@@ -76,6 +76,27 @@ __device__ __forceinline__ float3 normalize3(float3 a)
 }
 __device__ __forceinline__ float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
+// The farthest that a ray the capsule test counts as a hit passes from the segment:
+// the radius, and
+//  * 2^-16 of the largest magnitude involved, for the FP32 rounding of positions
+//    along the ray and of their projection (below 2^-20 of it for cameras within 64
+//    scene sizes);
+//  * what the test's discriminants lose by cancellation.  They compare a squared
+//    distance with the radius squared after subtracting terms of up to the length
+//    squared.  With u = 2^-24 the sphere at the far end loses 3 u in |oc|^2, 6 u in
+//    (d . oc)^2, 7 u through |d| <> 1 and 3 u in oc itself, about 19 u of the length
+//    squared, and the cylinder's terms about as much; 2^-19 = 32 u covers both.  (The
+//    largest found on 2e8 hits, segments of 0.1 to 8 units and radii of 1e-6 to 0.03 at
+//    every angle to the ray: 8.4 u.)  Nothing for a curve's short segments (10 radii:
+//    1e-4 of the radius), several radii for the thinnest (1e4 radii long: 14).
+__device__ __forceinline__ float capsule_reach(float4 a, float4 b, float radius, float magnitude)
+{
+  const float3 ba = sub3(xyz(b), xyz(a));
+  float reach;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(reach) : "f"(radius * radius + dot3(ba, ba) * 0x1p-19f));
+  return fmaxf(reach, radius) + (radius + magnitude) * (1.0f / 65536.0f);
+}
+
 // Order-preserving map of a float to an unsigned integer (for atomicMin/Max).
 __device__ __forceinline__ unsigned int float_key(float f)
 {
@@ -551,14 +572,13 @@ __device__ float3 shade(const render_args& A, float3 o, float3 d, const hit_reco
 // most tests are skipped whatever the order of the capsules.
 //
 // The rectangle is conservative: camera-space bounds of the segment, grown by
-// the radius and by 2^-16 of the largest magnitude involved (FP32 rounding of the
-// projection and of the capsule test is below 2^-20 of it for cameras within 64
-// scene sizes), plus 1/16 pixel.
+// its reach (capsule_reach), plus 1/16 pixel.
 struct raster_args
 {
   int              width, height;
   float3           origin, right, up, forward;   // orthonormal camera basis (right: +x, up: rows from the top)
   float            focal;                        // pixels per unit of slope
+  float            half_inverse_focal2;          // 0.5 / focal^2
   const float4*    vertices;
   const long long* prim_vertex;
   long long        prims;
@@ -604,7 +624,7 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
 {
   const float3 a = sub3(xyz(a4), A.origin), b = sub3(xyz(b4), A.origin);
   const float magnitude = fmaxf(fmaxf(largest3(a4), largest3(b4)), fmaxf(fmaxf(fabsf(A.origin.x), fabsf(A.origin.y)), fabsf(A.origin.z)));
-  const float pad = A.radius + (A.radius + magnitude) * (1.0f / 65536.0f);
+  const float pad = capsule_reach(a4, b4, A.radius, magnitude);
   const float za = dot3(a, A.forward), zb = dot3(b, A.forward);
   const float z0 = fminf(za, zb) - pad, z1 = fmaxf(za, zb) + pad;
   screen_rect r {0, 0, 0, 0, z0, {0.0f, 0.0f}, {0.0f, 0.0f}, INFINITY, false};
@@ -636,8 +656,8 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   const float ia = __fdividef(A.focal, za), ib = __fdividef(A.focal, zb);
   r.from = make_float2(cx + xa * ia - float(x0), cy - ya * ia - float(y0));
   r.along = make_float2(cx + xb * ib - float(x0) - r.from.x, cy - yb * ib - float(y0) - r.from.y);
-  const float sx = __fdividef(fmaxf(fabsf(x_lo), fabsf(x_hi)), z0), sy = __fdividef(fmaxf(fabsf(y_lo), fabsf(y_hi)), z0);
-  const float reach = pad * i0 * (1.0001f + 0.5f * (sx * sx + sy * sy)) + 0.0625f;
+  const float ex = fmaxf(fabsf(x_lo), fabsf(x_hi)) * i0, ey = fmaxf(fabsf(y_lo), fabsf(y_hi)) * i0;   // slope x focal
+  const float reach = pad * i0 * (1.0001f + (ex * ex + ey * ey) * A.half_inverse_focal2) + 0.0625f;
   r.radius2 = reach * reach;
   return r;
 }
@@ -1299,6 +1319,7 @@ bool render_raster(pars_gpu_context& ctx, render_state& r, const render_args& A)
   R.up = make_float3(r.above[0], r.above[1], r.above[2]);
   R.forward = make_float3(r.ahead[0], r.ahead[1], r.ahead[2]);
   R.focal = r.focal;
+  R.half_inverse_focal2 = float(0.5 / (double(r.focal) * r.focal));
   R.vertices = r.vertices;
   R.prim_vertex = r.prim_vertex.as<const long long>();
   R.prims = r.prims;
