@@ -189,8 +189,8 @@ __global__ void leaf_first_kernel(const int* __restrict__ flags, const long long
   if (k < prims && flags[k]) first[index[k]] = k;
 }
 
-// Leaf boxes (the union of the leaf's capsule boxes, padded so that a hit
-// computed in FP32 lies strictly inside it) and Morton keys of the box
+// Leaf boxes (the union of the leaf's capsule boxes, padded by the capsules' reach
+// so that a hit computed in FP32 lies inside it) and Morton keys of the box
 // centres; run[l] = the leaf's packed first start vertex and segment count.
 __global__ void leaf_kernel(const float4* __restrict__ vertices, const long long* __restrict__ prim_vertex, long long prims,
                             const long long* __restrict__ first, long long leaves, float radius,
@@ -205,13 +205,15 @@ __global__ void leaf_kernel(const float4* __restrict__ vertices, const long long
   const long long g = prim_vertex[f];
   float4 v = vertices[g];
   float3 lo = make_float3(v.x, v.y, v.z), hi = lo;
+  float pad = 0.0f;
   for (long long s = 1; s <= count; ++s)
   {
+    const float4 before = v;
     v = vertices[g + s];
+    pad = fmaxf(pad, capsule_reach(before, v, radius, key_float(bounds[6])));
     lo = make_float3(fminf(lo.x, v.x), fminf(lo.y, v.y), fminf(lo.z, v.z));
     hi = make_float3(fmaxf(hi.x, v.x), fmaxf(hi.y, v.y), fmaxf(hi.z, v.z));
   }
-  const float pad = radius + (radius + key_float(bounds[6])) * (1.0f / 65536.0f);
   leaf_lo[l] = make_float4(lo.x - pad, lo.y - pad, lo.z - pad, 0.0f);
   leaf_hi[l] = make_float4(hi.x + pad, hi.y + pad, hi.z + pad, 0.0f);
   run[l] = g | ((count - 1) << 56);
@@ -435,10 +437,10 @@ __device__ __forceinline__ void leaf_test(const render_args& A, float3 o, float3
   const int count = RUNS ? int(packed >> 56) + 1 : 1;
   float4 a = A.vertices[g];
   if (count == 1) { capsule_test(o, d, a, A.vertices[g + 1], A.radius, g, best); return; }
-  const float pad = A.radius + (A.radius + key_float(A.bounds[6])) * (1.0f / 65536.0f);
   for (int s = 0; s < count; ++s)
   {
     const float4 b = A.vertices[g + s + 1];
+    const float pad = capsule_reach(a, b, A.radius, key_float(A.bounds[6]));
     float tn;
     if (box_hit(o, inv, fminf(a.x, b.x) - pad, fminf(a.y, b.y) - pad, fminf(a.z, b.z) - pad, fmaxf(a.x, b.x) + pad,
                 fmaxf(a.y, b.y) + pad, fmaxf(a.z, b.z) + pad, best.t, tn))
