@@ -79,6 +79,30 @@ private:
   std::size_t bytes_ = 0;
 };
 
+// Counters that the host reads while the stream goes on: page-locked words (a copy
+// into pageable memory makes the host wait for all that the stream holds), and the
+// event behind the copy.
+struct host_counts
+{
+  static constexpr int count = 4;
+  unsigned long long*  words  = nullptr;
+  cudaEvent_t          copied = nullptr;
+
+  host_counts() = default;
+  host_counts(const host_counts&) = delete;
+  host_counts& operator=(const host_counts&) = delete;
+  ~host_counts()
+  {
+    if (copied) cudaEventDestroy(copied);
+    if (words) cudaFreeHost(words);
+  }
+  void create()
+  {
+    if (!words) PARS_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&words), sizeof(unsigned long long) * count, cudaHostAllocDefault));
+    if (!copied) PARS_CUDA(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
+  }
+};
+
 struct field_entry
 {
   device_buffer data;          // float4 [slices][X][Y][Z]
@@ -188,6 +212,7 @@ struct render_state
   long long     frames = 0;
   device_buffer accum, jitter, status, image, thresholds;
   device_buffer directions, pixel_keys, raster_count, raster_slices;   // capsules onto the screen: rays, closest hits, pixels covered
+  host_counts   counted;                          // raster_count as the host reads it
   float         srgb_thresholds[255];
 };
 
