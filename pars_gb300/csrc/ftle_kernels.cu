@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(co
   const unsigned lanes_below = (1u << lane) - 1u;
   long long pool_next = 0, pool_end = 0;   // warp-uniform
   bool exhausted = false, alive = false, ended = false;   // ended: holds a particle not yet written
-  unsigned int steps = 0;                  // this lane's steps, all its particles
+  unsigned int steps = 0;                  // this lane's steps, those not yet added to a.steps
   long long out = 0;                       // the particle's voxel, -1: none
   int it = 1;
   float4 pos = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -112,6 +112,8 @@ __global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(co
         // seed position here.
         if constexpr (SCHEME != flow_frozen) { if (it > 1) pos = flow_position(a.f, q); }
         if (out >= 0) a.flow[out] = pos;
+        // (a lane takes particle after particle, and the warp's sum has 32 bits)
+        if (steps >> 26) { atomicAdd(a.steps, (unsigned long long)steps); steps = 0; }
         ended = false;
       }
       while (need && !exhausted)
