@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(128) trace_persistent_kernel(const __grid_cons
 // 512^3, 1 M seeds, the whole call: 22.8, 19.1, 12.5 ms.
 constexpr int async_ahead = 16;
 constexpr unsigned int async_sleep = 8192;
-constexpr unsigned int async_wait_limit = 1u << 20;   // warp-wide idle polls (about 10 s with the pauses)
+constexpr unsigned int async_max_polls = 1u << 20;    // warp-wide idle polls (about 10 s with the pauses)
 
 // Device-scope memory-model accesses (PTX ld.acquire / ld.relaxed /
 // st.release): a segment's record is written before its ready flag is
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(128) async_trace_kernel(const __grid_constant_
     {
       // nothing to trace: stop on another lane's failure or after the wait limit
       if (load_acquire(a.error) != async_ok) break;
-      if (++waits > async_wait_limit) { if (lane == 0) atomicCAS(a.error, async_ok, async_wait_limit); break; }
+      if (++waits > async_max_polls) { if (lane == 0) atomicCAS(a.error, async_ok, async_wait_limit); break; }
       // (idle warps that poll without a pause load the counters' L2 slice, and
       // every lane that looks for a continuation waits for it)
       __nanosleep(min(async_sleep, 256u << min(waits - 1, 8u)));
