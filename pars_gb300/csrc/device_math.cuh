@@ -409,14 +409,18 @@ __device__ __forceinline__ float4 frozen_step(const step_rule& r, const float4& 
 // hi + lo carries the position to about twice FP32 precision.  Small steps
 // added to positions of order one otherwise lose a correlated fraction of an
 // ulp every step.
-__device__ __forceinline__ void compensated_add(float& hi, float& lo, float delta)
+__device__ __forceinline__ void compensated_take(float& hi, float& lo, float d)
 {
-  const float d = delta + lo;
   const float s = hi + d;
   const float bp = s - hi;
   lo = (hi - (s - bp)) + (d - bp);
   hi = s;
 }
+__device__ __forceinline__ void compensated_add(float& hi, float& lo, float delta) { compensated_take(hi, lo, delta + lo); }
+// The same with delta = a b, the product not rounded before it is added to lo.  Said
+// explicitly: whether the compiler fuses `compensated_add(hi, lo, a * b)` depends on
+// the kernel around it, and the same step would have several roundings.
+__device__ __forceinline__ void compensated_add_product(float& hi, float& lo, float a, float b) { compensated_take(hi, lo, fmaf(a, b, lo)); }
 
 // Knuth's error-free TwoSum: s = RN(a + b) and e = (a + b) - s exactly.
 // Written with round-to-nearest intrinsics, which the compiler never fuses
@@ -850,9 +854,9 @@ __device__ __forceinline__ void local_step(const field_view& f, corner_cache& k,
   if constexpr (FETCH) fetch_cell(f, k, q, fmaf(h, k1.x, q.ux), fmaf(h, k1.y, q.uy), fmaf(h, k1.z, q.uz), slot);
   if (!rk4)
   {
-    compensated_add(q.ux, q.lx, h * k1.x);
-    compensated_add(q.uy, q.ly, h * k1.y);
-    compensated_add(q.uz, q.lz, h * k1.z);
+    compensated_add_product(q.ux, q.lx, h, k1.x);
+    compensated_add_product(q.uy, q.ly, h, k1.y);
+    compensated_add_product(q.uz, q.lz, h, k1.z);
     renormalize(q);
     return;
   }
@@ -912,9 +916,9 @@ __device__ __forceinline__ void local_unsteady_step(const field_view& f, const t
 {
   if (!rk4)
   {
-    compensated_add(q.ux, q.lx, h * k1.x);
-    compensated_add(q.uy, q.ly, h * k1.y);
-    compensated_add(q.uz, q.lz, h * k1.z);
+    compensated_add_product(q.ux, q.lx, h, k1.x);
+    compensated_add_product(q.uy, q.ly, h, k1.y);
+    compensated_add_product(q.uz, q.lz, h, k1.z);
     renormalize(q);
     return;
   }
@@ -999,9 +1003,9 @@ __device__ __forceinline__ void adams_step_local(const field_view& f, corner_cac
   local_position predicted = q;
   if (hist.started)
   {
-    compensated_add(predicted.ux, predicted.lx, h * fmaf(1.5f, k1.x, -0.5f * hist.v.x));
-    compensated_add(predicted.uy, predicted.ly, h * fmaf(1.5f, k1.y, -0.5f * hist.v.y));
-    compensated_add(predicted.uz, predicted.lz, h * fmaf(1.5f, k1.z, -0.5f * hist.v.z));
+    compensated_add_product(predicted.ux, predicted.lx, h, fmaf(1.5f, k1.x, -0.5f * hist.v.x));
+    compensated_add_product(predicted.uy, predicted.ly, h, fmaf(1.5f, k1.y, -0.5f * hist.v.y));
+    compensated_add_product(predicted.uz, predicted.lz, h, fmaf(1.5f, k1.z, -0.5f * hist.v.z));
     renormalize(predicted);
   }
   else
