@@ -67,7 +67,7 @@ __device__ __forceinline__ void flow_step(const flow_map_args& a, corner_cache& 
   else                                               tableau_step_local<SCHEME - flow_midpoint>(a.f, cache, a.rule.h, q, v);
 }
 
-// One particle per lane, and lanes whose particles have ended take the next
+// Maps of many steps: one particle per lane, and lanes whose particles have ended take the next
 // seeds of their warp's pool (refill_rule): particles leave the grid
 // after very different step counts, and with one seed per thread a warp's lanes
 // idled until its longest particle ended.  Warps take pools of 32 consecutive
@@ -177,28 +177,93 @@ __global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_kernel(co
   if (lane == 0 && warp_steps) atomicAdd(a.steps, (unsigned long long)warp_steps);
 }
 
+// One seed per thread, for maps of few steps: refilled lanes are out of step, and a
+// lane that ends between two looks idles until the next, which few steps do not make
+// up for.  200^3 Euler frozen, 11 / 29 / 49 / 81 steps, seeds from the counter against
+// this: 1028 / 2328 / 3881 / 5845 against 870 / 2082 / 3440 / 5599 us; 128^3, 129 steps:
+// 2182 against 2331.
+template <int SCHEME>
+__global__ void __launch_bounds__(128, flow_min_ctas(SCHEME)) flow_map_once_kernel(const __grid_constant__ flow_map_args a)
+{
+  const long long total = (long long)a.px * a.py * a.pz, s = (long long)blockIdx.x * 128 + threadIdx.x;
+  unsigned int steps = 0;
+  if (s < total)
+  {
+    int ix, iy, iz;
+    lattice_index(s, a.py, a.pz, ix, iy, iz);
+    float4 pos = make_float4(__fadd_rn(a.ox, __fmul_rn(a.sx, float(ix))), __fadd_rn(a.oy, __fmul_rn(a.sy, float(iy))),
+                             __fadd_rn(a.oz, __fmul_rn(a.sz, float(iz))), 0.0f);
+    corner_cache cache;
+    frozen_history hist = frozen_history();
+    if constexpr (SCHEME == flow_frozen)
+    {
+      for (int it = 1; it < a.iterations; ++it, ++steps)
+      {
+        float3 v;
+        if (!sample_inside_cached(a.f, cache, pos, v) || is_zero(v)) break;
+        pos = frozen_step(a.rule, pos, v, hist);
+      }
+    }
+    else
+    {
+      local_position q = to_local(a.f, pos);
+      for (int it = 1; it < a.iterations; ++it, ++steps)
+      {
+        if (!local_inside(a.f, q)) break;
+        const float3 v = sample_local(a.f, cache, q.ix, q.iy, q.iz, q.ux, q.uy, q.uz);
+        if (is_zero_local(a.f, v)) break;
+        flow_step<SCHEME>(a, cache, q, v, hist);
+      }
+      if (steps) pos = flow_position(a.f, q);   // (iterations <= 1: the seed position, as in flow_map_kernel)
+    }
+    if (ix < a.fx && iy < a.fy && iz < a.fz) a.flow[((long long)ix * a.fy + iy) * a.fz + iz] = pos;
+  }
+  const unsigned int warp_steps = __reduce_add_sync(0xffffffffu, steps);
+  if ((threadIdx.x & 31) == 0 && warp_steps) atomicAdd(a.steps, (unsigned long long)warp_steps);
+}
+
+const void* flow_map_once_kernels[flow_schemes] = {
+  (const void*)flow_map_once_kernel<flow_frozen>, (const void*)flow_map_once_kernel<flow_classic>,
+  (const void*)flow_map_once_kernel<flow_midpoint>, (const void*)flow_map_once_kernel<flow_cash_karp>,
+  (const void*)flow_map_once_kernel<flow_dormand_prince>, (const void*)flow_map_once_kernel<flow_fehlberg>,
+  (const void*)flow_map_once_kernel<flow_adams_bashforth>, (const void*)flow_map_once_kernel<flow_adams_moulton>};
+
 const void* flow_map_kernels[flow_schemes] = {
   (const void*)flow_map_kernel<flow_frozen>, (const void*)flow_map_kernel<flow_classic>, (const void*)flow_map_kernel<flow_midpoint>,
   (const void*)flow_map_kernel<flow_cash_karp>, (const void*)flow_map_kernel<flow_dormand_prince>,
   (const void*)flow_map_kernel<flow_fehlberg>, (const void*)flow_map_kernel<flow_adams_bashforth>,
   (const void*)flow_map_kernel<flow_adams_moulton>};
 
-// Resident CTAs of the kernel on the device, all SMs together.
+// Resident CTAs of the kernel on the device, all SMs together.  (Loads both kernels:
+// a later launch may be inside a stream capture.)
 cudaError_t flow_map_resident(flow_scheme scheme, int device, int* ctas)
 {
   int per_sm = 0, sms = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flow_map_kernels[scheme], 128, 0);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flow_map_once_kernels[scheme], 128, 0);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, flow_map_kernels[scheme], 128, 0);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   *ctas = std::max(1, per_sm) * std::max(1, sms);
   return e;
 }
 
-// The lattice's seeds (at least one) on at most `resident` CTAs.
+// The lattice's seeds (at least one) on at most `resident` CTAs that take them from the
+// counter, or each on its own thread.  With refilled lanes (six seeds a lane and more)
+// the two break even at about 100 steps: 128^3 Euler, midpoint and Adams-Bashforth
+// frozen are 1 to 3 % slower from the counter at 81 steps and 5 to 6 % faster at 129.
+// Below, warps run their seeds to the end either way, and the counter's trips show in
+// short launches only: 64^3, 4 steps 42 against 32 us, 11 to 39 steps within 3 %.
+constexpr int flow_once_refilled = 96, flow_once_whole = 16;
 cudaError_t launch_flow_map_kernel(const flow_map_args& a, flow_scheme scheme, int resident, cudaStream_t stream)
 {
   const long long total = (long long)a.px * a.py * a.pz;
-  const unsigned grid = (unsigned)std::min<long long>(resident, (total + 127) / 128);
   refill_rule refill = refill_for(total, resident * 128LL);
+  const long long ctas = (total + 127) / 128;
+  if (a.iterations <= (refill.lanes < 32 ? flow_once_refilled : flow_once_whole) && ctas < (1LL << 31))
+  {
+    void* args[] = {(void*)&a};
+    return cudaLaunchKernel(flow_map_once_kernels[scheme], (unsigned)ctas, 128, args, 0, stream);
+  }
+  const unsigned grid = (unsigned)std::min<long long>(resident, ctas);
   void* args[] = {(void*)&a, (void*)&refill};
   return cudaLaunchKernel(flow_map_kernels[scheme], grid, 128, args, 0, stream);
 }
