@@ -169,8 +169,13 @@ __device__ __forceinline__ void add_steps(const trace_launch& a, unsigned int st
 // FETCH (re-sampled RK4 on fields that do not stay in L2): a step's stages lie in
 // other cells, and each waits for its corners before the next is known; the end
 // cell's are fetched while the middle ones are sampled.
-template <int MODE, bool FETCH = false>
-__global__ void __launch_bounds__(32, 16) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
+// WARPS 20 (frozen steps, 96 registers): launches between the 16 and the 20 warps per SM
+// that one particle a lane needs.  In pools of the 16 that the persistent kernel holds
+// (111 registers) they waited for a second, nearly empty wave: 84000 Euler curves of 150
+// steps, 64^3 / 160^3: 399 / 457 us, now 279 / 317 (359 / 405 when the persistent kernel
+// had 95 registers; bounding it to them now costs 99000 to 200000 curves 2 to 6 %).
+template <int MODE, bool FETCH = false, int WARPS = 16>
+__global__ void __launch_bounds__(32, WARPS) trace_kernel(const __grid_constant__ trace_launch a, int lanes)
 {
   unsigned int slot = 0;
   if constexpr (FETCH)
@@ -731,13 +736,20 @@ void launch_trace(pars_gpu_context& ctx, const trace_launch& a)
   if (per_sm < 0) PARS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent, 128, 0));
   const int sms = ctx.sm_count;
   const long long resident_warps = (long long)std::max(per_sm, 1) * sms * 4;
+  // one particle per thread while all of them are resident
+  constexpr int frozen_warps = 20;
+  const bool one_each = a.count <= 32 * std::max(resident_warps, mode == trace_frozen ? (long long)frozen_warps * sms : 0LL);
   launch_scope scope(ctx, "trace_streamlines");
-  if (a.count <= resident_warps * 32)
+  if (one_each)
   {
-    // one particle per thread, one warp per CTA so that the work spreads over all SMs
+    // one warp per CTA so that the work spreads over all SMs
     const int lanes = narrow_lanes(a.count, sms);
     const unsigned grid = (unsigned)((a.count + lanes - 1) / lanes);
-    if (mode == trace_frozen)       trace_kernel<trace_frozen><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    if (mode == trace_frozen)
+    {
+      if (a.count <= 32LL * 16 * sms) trace_kernel<trace_frozen><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+      else trace_kernel<trace_frozen, false, frozen_warps><<<grid, 32, 0, ctx.stream>>>(a, lanes);
+    }
     else if (mode == trace_classic)
     {
       // 10648 particles, 1000 RK4 steps on a 124 MB field: 1622 us, 1448 with the
