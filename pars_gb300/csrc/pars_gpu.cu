@@ -889,9 +889,10 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
   cudaEvent_t a, b;
   PARS_CUDA(cudaEventCreate(&a));
   PARS_CUDA(cudaEventCreate(&b));
-  std::vector<float> fastest(batch_variant_count(), 0.0f);
+  std::vector<float> fastest(batch_variant_count(), INFINITY);
   for (int v = 0; v < batch_variant_count(); ++v)
   {
+    if (c == batch_unsteady && v == batch_unsteady_few) continue;   // chosen by the seeds (batch_shape)
     for (int rep = 0; rep < 2; ++rep)
     {
       PARS_CUDA(cudaMemcpyAsync(device_jobs, jobs.data(), sizeof(batch_job_device) * count, cudaMemcpyHostToDevice, ctx.stream));
@@ -913,7 +914,6 @@ void tune_class(pars_gpu_context& ctx, int c, std::vector<batch_job_device> jobs
   // resident warps per SM (on the 256^3 flow map the 96-register shape, five
   // CTAs of 128, beats the 104-register ones by 7 %, which the probes alone
   // do not resolve reliably).
-  if (c == batch_unsteady) fastest[batch_unsteady_few] = INFINITY;   // chosen by the seeds (batch_shape)
   const float best_time = *std::min_element(fastest.begin(), fastest.end());
   int best_v = -1, best_warps = -1;
   for (int v = 0; v < batch_variant_count(); ++v)
