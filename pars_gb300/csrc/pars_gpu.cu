@@ -1115,7 +1115,6 @@ long long engine_submit(pars_gpu_context& ctx, const batch_job_device& job)
   batch_job_device j = job;
   j.clock = make_slice_clock(j.time, j.time_begin, j.rule.h);
   if (ctx.batch_variant[c] < 0) tune_class(ctx, c, {j});
-  if (E.open == 0) E.variant = batch_shape(ctx, c, j.seed_count);   // fixed while the class has work
   engine_reserve(ctx, E, int(E.jobs.size()) + 1);
   j.first_pool = E.total_pools;
   j.steps = E.counters.as<unsigned long long>() + 4 + E.jobs.size();
@@ -1168,10 +1167,18 @@ std::vector<std::pair<long long, unsigned long long>> engine_advance(pars_gpu_co
         }
       E.uploaded = n;
     }
-    const long long resident = batch_horizon_warps(ctx, c, E.variant);
+    // The launch shape goes by the seeds of all open jobs.  A larger one may take over
+    // parked groups (each needs a warp of its own to resume it), so the group buffers
+    // are made for the most warps of any.
+    long long open_seeds = 0;
+    for (int k = 0; k < n; ++k) if (!E.complete[k]) open_seeds += E.jobs[k].seed_count;
+    const int shape = batch_shape(ctx, c, open_seeds);
+    if (E.parked == 0 || batch_horizon_warps(ctx, c, shape) >= batch_horizon_warps(ctx, c, E.variant)) E.variant = shape;
+    long long resident = 0;
+    for (int v = 0; v < batch_variant_count(); ++v) resident = std::max(resident, batch_horizon_warps(ctx, c, v));
     if (E.group_capacity < resident)
     {
-      PARS_REQUIRE(E.parked == 0, "the engine's launch shape changed while groups are parked");
+      PARS_REQUIRE(E.parked == 0, "parked groups in buffers that are too small");
       for (int b = 0; b < 2; ++b)
       {
         E.groups[b].reserve(sizeof(batch_parked_group) * resident);
