@@ -189,6 +189,7 @@ struct render_state
   float         radius = 1.0f;
   long long     curves_generation = -1;         // >= 0: the context's curves at that generation
   device_buffer own_vertices, own_colors, prim_vertex, batch_bounds;
+  bool          drawn = false;                  // the scene has been drawn onto the screen since it was set
   // BVH (linear, Karras 2012)
   bool          tree_valid = false;
   bool          status_pending = false;         // the build's status word is not read yet

@@ -586,14 +586,16 @@ struct raster_args
   long long        prims;
   float            radius;
   const float2*    jitter;                       // of the frames of this call
-  int              frame;
-  const float4*    directions;                   // this frame's ray of each pixel
-  unsigned long long* keys;                      // per pixel
+  int              frame;                        // the launch's first; the others follow by blockIdx.y
+  const float4*    directions;                   // the ray of each pixel, frame by frame
+  unsigned long long* keys;                      // per pixel, frame by frame
   unsigned long long* count;                     // [0] rectangle pixels of all capsules, [1] of the largest, [2] bits of
                                                  // the largest |coordinate|, [3] slices of large rectangles
   uint2*           slices;                       // of the large rectangles: capsule, slice
   unsigned long long  limit;                     // beyond it, or with a larger rectangle, the tree is the cheaper way:
   unsigned int        limit_each;                // nothing is drawn
+  float            large;                        // pixels from which a capsule is drawn in slices
+  unsigned int     share;                        // capsules that a warp takes at a time
 };
 
 struct screen_rect
@@ -611,6 +613,8 @@ struct screen_rect
 // up to a pixel.  So a capsule is large or not by its extent before the jitter, and a
 // large one is drawn through the rectangle of all jitters in every frame.
 constexpr int raster_slice = 2048, raster_slices = 1 << 16;
+constexpr long long raster_few = 16384;       // capsules that need small parts to fill the GPU
+constexpr long long raster_stack = 1 << 21;   // pixels of the frames that go through one launch together
 
 __device__ __forceinline__ float largest3(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
 
@@ -644,7 +648,7 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   auto first = [&](float c, float v, int size) { return int(fminf(fmaxf(ceilf(c + v - margin(v)), 0.0f), float(size))); };
   auto last = [&](float c, float v, int size) { return int(fmaxf(fminf(floorf(c + v + margin(v)), float(size - 1)), -1.0f)); };
   int x0 = first(cx, left, A.width), x1 = last(cx, right, A.width), y0 = first(cy, top, A.height), y1 = last(cy, bottom, A.height);
-  r.large = !((right - left) * (bottom - top) <= float(raster_slice));
+  r.large = !((right - left) * (bottom - top) <= A.large);
   if (r.large)
   {
     // of every jitter in [0, 1] (each operation is monotone, so it holds this one's)
@@ -768,23 +772,24 @@ __device__ __forceinline__ float3 pixel_ray(const render_args& A, int px, int py
                                 A.corner.z + sx * A.du.z + sy * A.dv.z));
 }
 
-// One frame's rays, and the keys of pixels without a hit.
+// The frames' rays, and the keys of pixels without a hit.
 __global__ void __launch_bounds__(256) raster_begin_kernel(const __grid_constant__ render_args A, const __grid_constant__ raster_args R,
                                                            float4* __restrict__ directions)
 {
   if (!raster_applies(R, R.count)) return;
-  const float2 jitter = R.jitter[R.frame];
+  const float2 jitter = R.jitter[R.frame + blockIdx.y];
   const int pixels = A.width * A.height;
+  const long long frame = (long long)blockIdx.y * pixels;
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < pixels; p += gridDim.x * blockDim.x)
   {
     const int py = p / A.width, px = p - py * A.width;
     const float3 d = pixel_ray(A, px, py, jitter);
-    directions[p] = make_float4(d.x, d.y, d.z, 0.0f);
-    R.keys[p] = ~0ULL;
+    directions[frame + p] = make_float4(d.x, d.y, d.z, 0.0f);
+    R.keys[frame + p] = ~0ULL;
   }
 }
 
-// A warp takes 32 capsules at a time: each lane projects one, the covered ones are
+// A warp takes up to 32 capsules at a time: each lane projects one, the covered ones are
 // packed into shared memory, and the lanes then walk the pixels of all their
 // rectangles together, 32 per turn.  A turn's capsules are found from a mask of
 // the rectangles that start in it.  Pixels too far from the projected segment, or
@@ -797,6 +802,12 @@ __global__ void __launch_bounds__(256) raster_begin_kernel(const __grid_constant
 // rectangles with two 758; tiny capsules (26.5 M on 960 x 540) do best with
 // rectangles and single turns: 407 us, 446 through the bands.  Limited by the keys'
 // latency at 32 warps per SM (64 registers; 48 registers 738, 72 registers 892).
+// Few capsules: as many warps as with many share them (R.share), rectangles from 256
+// pixels on are cut into slices, and slices into parts of down to 128 pixels, because
+// a slice of 2048 pixels is 75 us of one warp.  1000 thick capsules on 1080 x 1920 /
+// 960 x 540 / from inside: 15.5 / 2.0 / 4.2 ms when 32 to a warp on four CTAs, now 0.27 /
+// 0.08 / 0.07.  Small images: the frames of a call side by side (blockIdx.y), 64 frames
+// of 100 capsules on 70 x 41: 3990 -> 91 us, 376 by the tree.
 __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_constant__ raster_args A)
 {
   if (!raster_applies(A, A.count)) return;
@@ -816,8 +827,8 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned lanes_below = (1u << lane) - 1u;
   uint2* queue = queues[warp];
-  const float2 jitter = A.jitter[A.frame];
-  const long long warps = (long long)gridDim.x * (raster_threads / 32);
+  const float2 jitter = A.jitter[A.frame + blockIdx.y];
+  const unsigned int warps = gridDim.x * (raster_threads / 32), prims = (unsigned int)A.prims;   // prims: below 2^31
 
   auto test = [&](uint2 item) {
     const entry& E = entries[warp][item.x];
@@ -841,7 +852,7 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
     E.inverse_w = __frcp_rn(float(band.w));
     E.w = band.w;
     E.start = start;
-    E.pixel = r.y0 * A.width + r.x0;
+    E.pixel = (int(blockIdx.y) * A.height + r.y0) * A.width + r.x0;   // (a launch's frames have 2^24 pixels at most)
     if constexpr (decltype(bands)::value)
     {
       E.across = band.columns ? r.h : r.w;
@@ -918,13 +929,13 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
     __syncwarp();                                  // before the next capsules take the shared memory
   };
 
-  for (long long first = ((long long)blockIdx.x * (raster_threads / 32) + warp) * 32; first < A.prims; first += warps * 32)
+  for (unsigned int first = (blockIdx.x * (raster_threads / 32) + warp) * A.share; first < prims; first += warps * A.share)
   {
-    const long long k = first + lane;
+    const unsigned int k = first + lane;
     screen_rect r {0, 0, 0, 0, 0.0f, {0.0f, 0.0f}, {0.0f, 0.0f}, 0.0f, false};
     float4 a, b;
     long long g = 0;
-    if (k < A.prims)
+    if (lane < A.share && k < prims)
     {
       g = A.prim_vertex[k];
       a = A.vertices[g];
@@ -955,17 +966,20 @@ __global__ void __launch_bounds__(raster_threads, 4) raster_kernel(const __grid_
     if (bands) draw(std::true_type {});
     else draw(std::false_type {});
   }
-  const int slices = int(A.count[3]);
-  for (long long s = (long long)blockIdx.x * (raster_threads / 32) + warp; s < slices; s += warps)
+  // few slices are cut once more, so that every warp gets a part
+  const unsigned int slices = (unsigned int)A.count[3];   // at most raster_slices
+  int cut = 0;
+  while (cut < 4 && slices << (cut + 1) <= warps) ++cut;
+  for (unsigned int s = blockIdx.x * (raster_threads / 32) + warp; s < slices << cut; s += warps)
   {
-    const uint2 slice = A.slices[s];
+    const uint2 slice = A.slices[s >> cut];
     const long long g = A.prim_vertex[slice.x];
     const float4 a = A.vertices[g], b = A.vertices[g + 1];
     const screen_rect r = project_capsule(A, a, b, jitter);
     if (lane == 0) place(std::true_type {}, 0, g, a, b, r, screen_band {0, r.w, 0.0f, 0.0f}, 0);
     __syncwarp();
-    const int begin = int(slice.y) * raster_slice;
-    walk(std::true_type {}, begin, min(begin + raster_slice, r.w * r.h), 1);
+    const int begin = int(slice.y) * raster_slice + (int(s) & ((1 << cut) - 1)) * (raster_slice >> cut);
+    walk(std::true_type {}, begin, min(begin + (raster_slice >> cut), r.w * r.h), 1);
   }
 }
 
@@ -1007,8 +1021,9 @@ __global__ void __launch_bounds__(render_tile * render_tile, HITS == hits_leaves
     hit_record h {INFINITY, LLONG_MAX, -1};
     if constexpr (HITS == hits_keys)
     {
-      d = xyz(__ldg(R.directions + pixel));
-      const unsigned long long key = R.keys[pixel];
+      const long long at = (long long)f * A.width * A.height + pixel;
+      d = xyz(__ldg(R.directions + at));
+      const unsigned long long key = R.keys[at];
       if (key != ~0ULL)
       {
         // the hit's distance and part, as the key's test found them
@@ -1291,6 +1306,7 @@ void render_use_spans(pars_gpu_context& ctx, render_state& r, const float4* vert
   PARS_CUDA(cudaGetLastError());
   r.curves_generation = -1;
   r.tree_valid = false;
+  r.drawn = false;
   render_clear(r);
 }
 
@@ -1334,8 +1350,9 @@ bool raster_fits(const render_state& r)
 bool render_raster(pars_gpu_context& ctx, render_state& r, const render_args& A)
 {
   const long long pixels = (long long)r.width * r.height;
-  r.directions.reserve(sizeof(float4) * pixels);
-  r.pixel_keys.reserve(sizeof(unsigned long long) * pixels);
+  const int stack = int(std::min<long long>(A.frames, std::max<long long>(1, raster_stack / pixels)));
+  r.directions.reserve(sizeof(float4) * pixels * stack);
+  r.pixel_keys.reserve(sizeof(unsigned long long) * pixels * stack);
   r.raster_count.reserve(sizeof(unsigned long long) * 4);
   r.raster_slices.reserve(sizeof(uint2) * raster_slices);
   if (ctx.sm_count <= 0) PARS_CUDA(cudaDeviceGetAttribute(&ctx.sm_count, cudaDevAttrMultiProcessorCount, ctx.device));
@@ -1363,9 +1380,16 @@ bool render_raster(pars_gpu_context& ctx, render_state& r, const render_args& A)
   // raster against build + walk: 520 k capsules covering 11 / 38 / 126 / 449 M
   // pixels 0.20 / 0.56 / 0.99 / 3.06 ms against 0.94 / 1.49 / 0.78 / 1.03 ms; 10 M
   // capsules covering 122 / 568 M 0.91 / 2.75 ms against 5.56 / 8.73 ms.
-  const double walk = 20.0 * double(pixels) + 30.0 * double(r.prims), build = 10.0 * double(pixels) + 27.0 * double(r.prims);
+  // Scenes of few capsules: the walk is shorter (960 x 540, camera inside: 10 us for 100
+  // capsules, 18 for 1000, 240 for 51 k), the build takes 75 us whatever their number.
+  // A scene that was drawn before is being looked at: its tree would serve the later
+  // views too, and is built where the drawing is slower than the walk alone.
+  const bool few = r.prims <= raster_few;
+  const double walk = few ? 20.0 * double(pixels) * std::min(1.0, std::sqrt(double(r.prims) / 5000.0)) : 20.0 * double(pixels) + 30.0 * double(r.prims);
+  const double build = r.drawn ? 0.0 : few ? 12e6 : 10.0 * double(pixels) + 27.0 * double(r.prims);
   R.limit = (unsigned long long)(walk + build / double(A.frames));
   R.limit_each = 1 << 20;
+  R.large = few ? 256.0f : float(raster_slice);
   PARS_CUDA(cudaMemsetAsync(R.count, 0, sizeof(unsigned long long) * 4, ctx.stream));
   {
     launch_scope scope(ctx, "raster_count");
@@ -1379,19 +1403,23 @@ bool render_raster(pars_gpu_context& ctx, render_state& r, const render_args& A)
   r.counted.create();
   PARS_CUDA(cudaMemcpyAsync(r.counted.words, R.count, sizeof(unsigned long long) * host_counts::count, cudaMemcpyDeviceToHost, ctx.stream));
   PARS_CUDA(cudaEventRecord(r.counted.copied, ctx.stream));
-  const unsigned int blocks = std::min<unsigned int>(blocks_for(r.prims, raster_threads), sms * 8u);
   render_args one = A;
-  one.frames = 1;
-  for (int f = 0; f < A.frames; ++f)
+  for (int f = 0; f < A.frames; f += one.frames)
   {
+    one.frames = std::min(stack, A.frames - f);
+    const unsigned int frames = (unsigned int)one.frames;
     R.frame = f;
     {
       launch_scope scope(ctx, "raster_begin");
-      raster_begin_kernel<<<std::min<unsigned int>(blocks_for(pixels, 256), sms * 8u), 256, 0, ctx.stream>>>(A, R, r.directions.as<float4>());
+      raster_begin_kernel<<<dim3(std::min<unsigned int>(blocks_for(pixels, 256), sms * 8u), frames), 256, 0, ctx.stream>>>(A, R, r.directions.as<float4>());
     }
+    // (fewer capsules a warp where that gives every warp some)
+    const unsigned int blocks = (sms * 8u + frames - 1) / frames;
+    R.share = 1;
+    while (R.share < 32 && 2 * R.share * (blocks * (raster_threads / 32)) <= r.prims) R.share *= 2;
     {
       launch_scope scope(ctx, "raster");
-      raster_kernel<<<blocks, raster_threads, 0, ctx.stream>>>(R);
+      raster_kernel<<<dim3(blocks, frames), raster_threads, 0, ctx.stream>>>(R);
     }
     if (f == 0)
     {
@@ -1403,6 +1431,7 @@ bool render_raster(pars_gpu_context& ctx, render_state& r, const render_args& A)
     one.fresh = 0;
   }
   PARS_CUDA(cudaStreamSynchronize(ctx.stream));
+  r.drawn = true;
   return true;
 }
 }
@@ -1621,6 +1650,7 @@ int32_t pars_gpu_ray_tracer_set_integral_curves(pars_gpu_context* ctx, float rad
     pars::render_use_context_curves(*ctx, r);
     r.curves_generation = ctx->curves.generation;
     r.tree_valid = false;
+    r.drawn = false;
     pars::render_clear(r);
   });
 }
@@ -1674,6 +1704,7 @@ int32_t pars_gpu_ray_tracer_set_integral_curves_host(pars_gpu_context* ctx, int6
     r.radius = radius;
     r.curves_generation = -1;
     r.tree_valid = false;
+    r.drawn = false;
     pars::render_clear(r);
   });
 }

@@ -558,6 +558,7 @@ void render_request(pars_gpu_service& svc, pars_gpu_context& c, request& r, cons
   rs.vertices = rs.colors = nullptr;       // the store may go once the request lets go
   rs.prims = 0;
   rs.tree_valid = false;
+  rs.drawn = false;
 }
 
 std::size_t run_streamline_batch(pars_gpu_service& svc, pars_gpu_context& c, std::vector<std::shared_ptr<request>>& batch, int stage_mode)

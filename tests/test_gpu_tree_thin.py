@@ -25,9 +25,9 @@ def test_thin_segments_of_the_tree_equal_the_oracle(ctx, port, length, radius):
         ctx.profile_reset()
         ctx.profile_enable(True)
         ctx.ray_tracer_trace(1)
-        walked = ctx.profile_get("tree_hits")[1]
+        drawn, rendered = ctx.profile_get("raster")[1], ctx.profile_get("render")[1]
         ctx.profile_enable(False)
-        assert walked == 1
+        assert drawn == 0 and rendered == 1
         expected, _ = port.render(batches, radius, view(length), SIZE)
         diff = np.any(ctx.ray_tracer_serialize() != expected, axis=-1)
         assert not diff.any(), (seed, int(diff.sum()), np.argwhere(diff)[:3].tolist())
