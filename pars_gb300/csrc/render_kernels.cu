@@ -76,6 +76,11 @@ __device__ __forceinline__ float3 normalize3(float3 a)
 }
 __device__ __forceinline__ float3 xyz(float4 a) { return make_float3(a.x, a.y, a.z); }
 
+// The dot product where its rounding is covered by a margin, as in the projection (this
+// file's products and sums are not contracted): 3 instructions instead of 5.  Counting /
+// drawing 26.5 M tiny capsules on 960 x 540: 175 / 448 -> 163 / 437 us.
+__device__ __forceinline__ float dot3_fused(float3 a, float3 b) { return __fmaf_rn(a.x, b.x, __fmaf_rn(a.y, b.y, a.z * b.z)); }
+
 // The farthest that a ray the capsule test counts as a hit passes from the segment:
 // the radius, and
 //  * 2^-16 of the largest magnitude involved, for the FP32 rounding of positions
@@ -93,7 +98,7 @@ __device__ __forceinline__ float capsule_reach(float4 a, float4 b, float radius,
 {
   const float3 ba = sub3(xyz(b), xyz(a));
   float reach;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(reach) : "f"(radius * radius + dot3(ba, ba) * 0x1p-19f));
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(reach) : "f"(__fmaf_rn(dot3_fused(ba, ba), 0x1p-19f, radius * radius)));
   return fmaxf(reach, radius) + (radius + magnitude) * (1.0f / 65536.0f);
 }
 
@@ -632,12 +637,12 @@ __device__ __forceinline__ screen_rect project_capsule(const raster_args& A, flo
   const float3 a = sub3(xyz(a4), A.origin), b = sub3(xyz(b4), A.origin);
   const float magnitude = fmaxf(fmaxf(largest3(a4), largest3(b4)), fmaxf(fmaxf(fabsf(A.origin.x), fabsf(A.origin.y)), fabsf(A.origin.z)));
   const float pad = capsule_reach(a4, b4, A.radius, magnitude);
-  const float za = dot3(a, A.forward), zb = dot3(b, A.forward);
+  const float za = dot3_fused(a, A.forward), zb = dot3_fused(b, A.forward);
   const float z0 = fminf(za, zb) - pad, z1 = fmaxf(za, zb) + pad;
   screen_rect r {0, 0, 0, 0, z0, {0.0f, 0.0f}, {0.0f, 0.0f}, INFINITY, false};
   if (!(z1 > 0.0f)) return r;                                   // behind the camera
   if (!(z0 > 0.0f)) { r.w = A.width; r.h = A.height; r.large = true; return r; }   // around it
-  const float xa = dot3(a, A.right), xb = dot3(b, A.right), ya = dot3(a, A.up), yb = dot3(b, A.up);
+  const float xa = dot3_fused(a, A.right), xb = dot3_fused(b, A.right), ya = dot3_fused(a, A.up), yb = dot3_fused(b, A.up);
   const float i0 = __fdividef(A.focal, z0), i1 = __fdividef(A.focal, z1);   // (a few ulps: far inside the margins)
   const float x_lo = fminf(xa, xb) - pad, x_hi = fmaxf(xa, xb) + pad, y_lo = fminf(ya, yb) - pad, y_hi = fmaxf(ya, yb) + pad;
   // pixel px samples the slope (px + jitter.x - width / 2) / focal, rows downwards
