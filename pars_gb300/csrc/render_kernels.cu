@@ -1514,8 +1514,10 @@ void render_frames(pars_gpu_context& ctx, render_state& r, int iterations)
   const dim3 tile(render_tile, render_tile);
   raster_args R {};
   // (without a volume, shading in the walk's own launch saves the rays' and hits' way
-  // through memory: 52 k capsules from inside, 1080 x 1920, 435 -> 411 us)
-  if (keyed && r.has_volume)
+  // through memory: 52 k capsules from inside, 1080 x 1920, 767 -> 734 us; with one too, where
+  // the walk is short: 95 capsules and a 64^3 volume 966 -> 894, 1000 capsules 870 -> 833,
+  // the volume alone on 70 x 41, 64 frames, 824 -> 360)
+  if (keyed && r.has_volume && r.leaves > 2048)
   {
     r.directions.reserve(sizeof(float4) * pixels);
     r.pixel_keys.reserve(sizeof(unsigned long long) * pixels);
