@@ -666,7 +666,7 @@ int32_t pars_gpu_profile_get   (pars_gpu_context* context, const char* name, dou
 int32_t pars_gpu_launch_count  (pars_gpu_context* context, int64_t* launches);
 /* Gather-bandwidth calibration (no counterpart in the reference; the measured
  * ceilings for the advection kernels' roofline).  Times 16-byte non-coherent
- * loads, the instruction the kernels use for cell corners, into a zeroed
+ * loads, as the kernels use for a cell's corners at x, into a zeroed
  * device buffer of buffer_bytes (rounded down to a power of two, 4 KiB to
  * 64 GiB) on the context's stream.  pattern 0: each warp request reads 512
  * contiguous bytes at a random aligned offset; 1: each lane 16 bytes at its

@@ -1,10 +1,12 @@
 // Gather-bandwidth calibration: the measured ceilings the advection kernels'
 // corner gathers are judged against.
 //
-// The advection kernels read a field through 16-byte non-coherent loads
-// (ld.global.nc.v4.f32, one per cell corner).  Which memory level serves them
-// depends on the working set, so the ceiling is measured per level on the
-// device itself, with the same load instruction:
+// The advection kernels read a field through non-coherent loads, one per cell
+// corner: 16 bytes (ld.global.nc.v4.f32) at x and, as those bring the z components
+// at x + 1 along, 8 bytes (ld.global.nc.v2.f32) at x + 1.  Which memory level serves
+// them depends on the working set, so the ceiling is measured per level on the device
+// itself, with the 16-byte loads (a scattered warp request costs about the same
+// whatever its width, so fewer bytes per step are not as much less work):
 //   coalesced: each warp request reads 512 contiguous bytes (four 128-byte
 //              lines) at a random 512-byte-aligned offset: the most useful
 //              bytes the L1 data pipe can deliver per wavefront;
